@@ -3,12 +3,14 @@ encoding, HLL sketch and generators (CUDA library vs CPU oracle).
 Sort, partition, partition offsets, ordered dictionary codes and HLL
 registers-derived estimates are bit-exact; join pairs are bit-exact after
 canonical sort; hash dictionary codes are checked as a bijection."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
 import eiger_b200 as gx
 import oracle as O
-from tests.helpers import to_dev
+from tests.helpers import to_dev, to_dev_raw
 
 pytestmark = pytest.mark.gpu
 
@@ -68,6 +70,38 @@ def test_argsort_and_sort_column(n):
     assert np.array_equal(sk.cpu().numpy(), ek) and np.array_equal(idx.cpu().numpy(), ei)
     only = gx.sort_column(to_dev(k))
     assert np.array_equal(only.cpu().numpy(), ek)
+
+
+@pytest.mark.parametrize("n", [2, 8191, 8192, 8193, 2048 * 7, 2048 * 7 + 1, (1 << 19) - 1, 1 << 19, 5120 * 149 + 3])
+@pytest.mark.parametrize("kdt,vdt", [(np.int8, np.int64), (np.uint16, np.int32), (np.int32, np.int32),
+                                     (np.float32, np.int64), (np.int64, np.int64), (np.float64, np.int32)])
+def test_sort_one_cta_and_onesweep_edges(n, kdt, vdt):
+    # The one-CTA sort (up to 8192 rows) and the look-back passes at the edges
+    # of their tiles, from views that start on and off 16-byte boundaries, with
+    # keys whose digits vary, are all the same in some passes (skipped) or in
+    # all of them, as pairs and as row ids.
+    rng = np.random.default_rng(n)
+    full = rng.integers(0, 256, size=(n + 1) * np.dtype(kdt).itemsize, dtype=np.uint8).view(kdt)
+    if np.dtype(kdt).kind == "f":
+        full = (rng.integers(-500, 500, n + 1) / 8).astype(kdt)
+    few = rng.integers(0, 3, n + 1).astype(kdt)
+    val = np.arange(n + 1).astype(vdt)
+    for k in (full, few, np.full(n + 1, 7, kdt)):
+        dk, dv = to_dev(k), to_dev_raw(val).view(to_dev(val).dtype)
+        for off in (0, 1):
+            for desc in (False, True):
+                ko, vo = gx.OwnedColumn(), gx.OwnedColumn()
+                gx.check(gx.lib.gx_sort_column_pair(
+                    gx.ColumnView(dk.data_ptr(), n, gx._NP_TO_GX[np.dtype(kdt)], off),
+                    gx.ColumnView(dv.data_ptr(), n, gx._NP_TO_GX[np.dtype(vdt)], off), 0, -1, int(desc), None, 0,
+                    gx._stream_ptr(None), C.byref(ko), C.byref(vo)))
+                ek, ev = O.sort_pairs(k[off:off + n].copy(), val[off:off + n].copy(), 0, -1, desc)
+                assert np.array_equal(gx.owned_to_torch(ko).cpu().numpy().view(np.uint8), ek.view(np.uint8))
+                assert np.array_equal(gx.owned_to_torch(vo).cpu().numpy(), ev)
+        sk, idx = gx.argsort(dk)
+        ek, ei = O.sort_pairs(k, iota=True)
+        assert np.array_equal(sk.cpu().numpy().view(np.uint8), ek.view(np.uint8))
+        assert np.array_equal(idx.cpu().numpy(), ei)
 
 
 @pytest.mark.parametrize("kdt", [np.int32, np.int64])
