@@ -270,6 +270,34 @@ __global__ void __launch_bounds__(SCAN_NT) k_tile_scan(const int64_t* __restrict
     }
 }
 
+// The whole scan of up to SCAN_ONE counts in one CTA (out[n] = total): one
+// launch instead of four to seven, which is what a scan of a small call costs.
+constexpr int SCAN_ONE_NT = 1024, SCAN_ONE_IPT = 8;
+constexpr int64_t SCAN_ONE = 1 << 15;
+__global__ void __launch_bounds__(SCAN_ONE_NT) k_scan_one(const int64_t* __restrict__ in, int64_t n,
+                                                          int64_t* __restrict__ out) {
+    __shared__ int64_t sm[SCAN_ONE_NT / 32 + 1];
+    int64_t before = 0;
+    for (int64_t base = 0; base < n; base += SCAN_ONE_NT * SCAN_ONE_IPT) {
+        int64_t v[SCAN_ONE_IPT], local = 0, total;
+#pragma unroll
+        for (int k = 0; k < SCAN_ONE_IPT; ++k) {
+            const int64_t i = base + threadIdx.x * SCAN_ONE_IPT + k;
+            v[k] = i < n ? in[i] : 0;
+            local += v[k];
+        }
+        int64_t run = before + dev_::block_exclusive_sum<SCAN_ONE_NT>(local, sm, &total);
+#pragma unroll
+        for (int k = 0; k < SCAN_ONE_IPT; ++k) {
+            const int64_t i = base + threadIdx.x * SCAN_ONE_IPT + k;
+            if (i < n) out[i] = run;
+            run += v[k];
+        }
+        before += total;
+    }
+    if (threadIdx.x == 0) out[n] = before;
+}
+
 __global__ void k_set_last(const int64_t* __restrict__ tile_prefix, int64_t ntiles,
                            const int64_t* __restrict__ tile_sums, int64_t* __restrict__ out,
                            int64_t n) {
@@ -300,15 +328,16 @@ void exclusive_scan_i64(const int64_t* in, int64_t* out, int64_t n, cudaStream_t
         fill_u64(out, 0, 1, s);
         return;
     }
+    if (n <= SCAN_ONE) {
+        k_scan_one<<<1, SCAN_ONE_NT, 0, s>>>(in, n, out);
+        GX_LAUNCHED();
+        return;
+    }
     int64_t ntiles = ceil_div(n, SCAN_TILE);
     dbuf sums(ntiles * sizeof(int64_t), s), pref((ntiles + 1) * sizeof(int64_t), s);
     k_tile_sums<<<(unsigned)ntiles, SCAN_NT, 0, s>>>(in, n, sums.get<int64_t>());
     GX_LAUNCHED();
-    if (ntiles == 1) {
-        fill_u64(pref.get(), 0, 1, s);
-    } else {
-        exclusive_scan_i64(sums.get<int64_t>(), pref.get<int64_t>(), ntiles, s);
-    }
+    exclusive_scan_i64(sums.get<int64_t>(), pref.get<int64_t>(), ntiles, s);
     k_tile_scan<<<(unsigned)ntiles, SCAN_NT, 0, s>>>(in, n, pref.get<int64_t>(), out);
     GX_LAUNCHED();
     k_set_last<<<1, 32, 0, s>>>(pref.get<int64_t>(), ntiles, sums.get<int64_t>(), out, n);

@@ -6,7 +6,7 @@ import pytest
 
 import eiger_b200 as gx
 import oracle as O
-from tests.helpers import to_dev
+from tests.helpers import to_dev, to_dev_raw
 
 pytestmark = pytest.mark.gpu
 
@@ -73,3 +73,41 @@ def test_count_nonzero_and_validation():
         gx.select([x], [gx.predicate(3, gx.CMP_LT, 1)])  # column out of range
     with pytest.raises(gx.GxError):
         gx.select([x], [])  # no predicate
+
+
+@pytest.mark.parametrize("dt", [np.int8, np.uint8, np.int16, np.uint16, np.int32, np.uint32, np.int64, np.uint64])
+def test_integer_ranges_at_the_type_limits(dt):
+    # Literals at, just inside and beyond the column type's limits: the ranges
+    # that the comparisons become must neither wrap nor clip.
+    inf = np.iinfo(dt)
+    a = np.array([inf.min, inf.min + 1, 0, 1, inf.max - 1, inf.max] * 700, dt)[:4099]
+    wide = [int(x) for x in a]
+    lim = (0, 2**64 - 1) if inf.min == 0 else (-2**63, 2**63 - 1)
+    lits = sorted({lim[0], lim[1], inf.min, inf.min + 1, inf.max, inf.max - 1, max(inf.min - 1, lim[0]),
+                   min(inf.max + 1, lim[1]), 0, 1})
+    cols = [to_dev_raw(a)]
+    view = gx.ColumnView(cols[0].data_ptr(), len(a), gx._NP_TO_GX[np.dtype(dt)], 0)
+    py = {gx.CMP_LT: lambda x, l, h: x < l, gx.CMP_LE: lambda x, l, h: x <= l, gx.CMP_GT: lambda x, l, h: x > l,
+          gx.CMP_GE: lambda x, l, h: x >= l, gx.CMP_EQ: lambda x, l, h: x == l, gx.CMP_NE: lambda x, l, h: x != l,
+          gx.CMP_BETWEEN: lambda x, l, h: l <= x < h}
+    for op in range(7):
+        for lo in lits:
+            for hi in lits if op == gx.CMP_BETWEEN else [0]:
+                m = gx.select_to_bitmask([view], [gx.predicate(0, op, lo, hi)]).cpu().numpy().astype(bool)
+                assert np.array_equal(m, np.array([py[op](x, lo, hi) for x in wide])), (op, lo, hi)
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+def test_float_ranges_with_infinities_nan_and_zeros(dt):
+    vals = [-np.inf, -1.5, -0.0, 0.0, 1e-40, 2.0, np.inf, np.nan]
+    a = np.array(vals * 600, dt)[:4101]
+    d = to_dev(a)
+    for op in range(7):
+        for lo in [-np.inf, -1.5, -0.0, 0.0, 0.1, 2.0, np.inf, np.nan]:
+            for hi in [-np.inf, 0.0, 2.0, np.inf, np.nan] if op == gx.CMP_BETWEEN else [0.0]:
+                e = np_cmp(a.astype(np.float64), op, lo, hi)
+                p = gx.predicate(0, op)
+                p.lo_f, p.hi_f = lo, hi
+                assert np.array_equal(gx.select_to_bitmask([d], [p]).cpu().numpy().astype(bool), e), (op, lo, hi)
+                got = gx.select([d], [p]).to_numpy(0)
+                assert np.array_equal(got, a[e], equal_nan=True), (op, lo, hi)
