@@ -4,13 +4,15 @@
 // ready-dictionary overload (src/cuda/compress/dictionary_encode.cu:144-373,
 // src/cuda/compress/dictionary_encode_dict_ready.cu:16-82).  The reference
 // inserts row ids into a cuco set sized N/0.25 when no hint is given, writes
-// an int64 representative per row and gathers codes through it.  Here the
-// table holds the canonical key bits and their code directly:
-//   * hash encode: pass 1 inserts keys and hands each new key the next code
-//     (atomicAdd); pass 2 looks every row up and writes its code — no
-//     per-row int64 scratch;
-//   * order-preserving: pass 1 inserts keys, the distinct keys are compacted
-//     and radix-sorted, each key's slot receives its rank, pass 2 as above;
+// an int64 representative per row and gathers codes through it.  Here a table
+// slot holds the canonical key bits and their code side by side, so one access
+// yields both:
+//   * hash encode: one pass that inserts keys, hands each new key the next
+//     code (atomicAdd) and writes every row's code;
+//   * order-preserving: the same pass writes first-insert codes and lists the
+//     distinct keys in that order; the keys are radix-sorted and a second pass
+//     replaces each code by its key's rank (a gather from ndv entries instead
+//     of another table lookup);
 //   * ready dictionary: the dictionary's values are inserted with code =
 //     position (the smallest position wins for duplicated values); rows whose
 //     value is absent get INT32_MIN (gamax::sentinel<int32_t>()).
@@ -24,13 +26,18 @@
 namespace gx {
 namespace {
 
-constexpr uint64_t D_EMPTY4 = ~0ull;
-constexpr uint64_t D_EMPTY8 = 0x8000000000000000ull;
-constexpr uint64_t NO_CODE = ~0ull;
+// Slots.  4-byte keys: one word, key << 32 | code.  8-byte keys: a 16-byte
+// pair {key, code}.  All bits set is an empty slot in both, so one memset
+// clears a table; the 8-byte key of all ones lives in the extra slot `cap`,
+// told apart by its code alone.
+constexpr unsigned long long D_EMPTY = ~0ull;
+constexpr uint64_t NO_CODE = ~0ull;                 // key absent
+constexpr uint64_t PENDING = ~0ull - 1;             // key claimed, code not yet there
+constexpr uint32_t PENDING4 = 0xFFFFFFFEu;
+constexpr uint32_t D_WAIT_LIMIT = 1u << 16;
 
 struct dtable {
-    unsigned long long* keys;   // cap + 1 slots; slot cap = key equal to the empty marker
-    unsigned long long* codes;  // cap + 1
+    unsigned long long* w;
     uint64_t mask;
     int* overflow;
 };
@@ -46,83 +53,99 @@ __device__ __forceinline__ uint64_t dhash(uint64_t k) {
     return fmix64(k);
 }
 
-// Returns the slot index, inserting when `insert`; -1 when absent / overflow.
+// Code of key k when it sits, settled, in its home slot (one plain load),
+// else NO_CODE: a stale read only sends the row to the full walk.
 template <int KW>
-__device__ __forceinline__ int64_t d_find(const dtable& t, uint64_t k, bool insert, bool* inserted) {
-    const uint64_t EMPTY = KW == 4 ? D_EMPTY4 : D_EMPTY8;
-    *inserted = false;
-    if (KW == 8 && k == EMPTY) {
-        int64_t s = (int64_t)t.mask + 1;
-        if (insert) {
-            unsigned long long old = atomicCAS(&t.keys[s], (unsigned long long)EMPTY ^ 1ull, (unsigned long long)EMPTY);
-            *inserted = old == (EMPTY ^ 1ull);
-            return s;
-        }
-        return t.keys[s] == EMPTY ? s : -1;
+__device__ __forceinline__ uint64_t d_home(const dtable& t, uint64_t k) {
+    const uint64_t slot = dhash<KW>(k) & t.mask;
+    if constexpr (KW == 4) {
+        const unsigned long long c = t.w[slot];
+        return (uint32_t)(c >> 32) == (uint32_t)k && (uint32_t)c < PENDING4 ? (uint64_t)(uint32_t)c : NO_CODE;
+    } else {
+        const ulonglong2 c = reinterpret_cast<const ulonglong2*>(t.w)[slot];
+        return c.x == k && k != D_EMPTY && c.y < PENDING ? c.y : NO_CODE;
+    }
+}
+
+// Hands out the next code and lists its key.
+__device__ __forceinline__ uint64_t d_next(unsigned long long* counter, void* dkeys, int kw, uint64_t k) {
+    const unsigned long long c = atomicAdd(counter, 1ull);
+    if (dkeys) {
+        if (kw == 4) static_cast<unsigned*>(dkeys)[c] = (unsigned)k;
+        else static_cast<unsigned long long*>(dkeys)[c] = k;
+    }
+    return c;
+}
+
+// Code of key k, inserting it.  PENDING when another thread has claimed the
+// key and not yet published its code (the inserter may be a lane of the same
+// warp, which a spinning branch could hold back); NO_CODE when the walk ran
+// out (overflow set).
+template <int KW>
+__device__ __forceinline__ uint64_t d_insert(const dtable& t, uint64_t k, unsigned long long* counter, void* dkeys) {
+    if (KW == 8 && k == D_EMPTY) {
+        unsigned long long* code = t.w + 2 * (t.mask + 1) + 1;
+        unsigned long long c = *(volatile unsigned long long*)code;
+        if (c != NO_CODE) return c;
+        c = atomicCAS(code, NO_CODE, PENDING);
+        if (c != NO_CODE) return c;
+        c = d_next(counter, dkeys, KW, k);
+        *(volatile unsigned long long*)code = c;
+        return c;
     }
     uint64_t slot = dhash<KW>(k) & t.mask;
     for (uint64_t p = 0, lim = t.mask < GX_PROBE_LIMIT ? t.mask : GX_PROBE_LIMIT - 1; p <= lim; ++p) {
-        unsigned long long cur = ((volatile unsigned long long*)t.keys)[slot];
-        if (cur == k) return (int64_t)slot;
-        if (cur == EMPTY) {
-            if (!insert) return -1;
-            unsigned long long old = atomicCAS(&t.keys[slot], (unsigned long long)EMPTY, (unsigned long long)k);
-            if (old == EMPTY) { *inserted = true; return (int64_t)slot; }
-            if (old == k) return (int64_t)slot;
+        if constexpr (KW == 4) {
+            unsigned long long cur = ((volatile unsigned long long*)t.w)[slot];
+            if (cur == D_EMPTY) {
+                cur = atomicCAS(&t.w[slot], D_EMPTY, (unsigned long long)k << 32 | PENDING4);
+                if (cur == D_EMPTY) {
+                    const uint64_t c = d_next(counter, dkeys, KW, k);
+                    ((volatile unsigned long long*)t.w)[slot] = (unsigned long long)k << 32 | (uint32_t)c;
+                    return c;
+                }
+            }
+            if ((uint32_t)(cur >> 32) == (uint32_t)k) return (uint32_t)cur == PENDING4 ? PENDING : (uint64_t)(uint32_t)cur;
+        } else {
+            unsigned long long* s = t.w + 2 * slot;
+            unsigned long long cur = *(volatile unsigned long long*)s;
+            if (cur == D_EMPTY) {
+                cur = atomicCAS(s, D_EMPTY, (unsigned long long)k);
+                if (cur == D_EMPTY) {
+                    const uint64_t c = d_next(counter, dkeys, KW, k);
+                    ((volatile unsigned long long*)s)[1] = c;
+                    return c;
+                }
+            }
+            if (cur == k) {
+                const unsigned long long c = ((volatile unsigned long long*)s)[1];
+                return c == NO_CODE ? PENDING : c;
+            }
         }
         slot = (slot + 1) & t.mask;
     }
-    if (insert) atomicExch(t.overflow, 1);
-    return -1;
+    atomicExch(t.overflow, 1);
+    return NO_CODE;
 }
 
-// Rows per thread per round of the insert and lookup kernels: their keys are
-// loaded, then their home slots probed, all at once, so each thread keeps
-// DU independent table reads in flight instead of one dependent chain.
-constexpr int DU = 4;
-
-// Slot of key k when it sits in its home slot (one plain load), else -1.
-// A stale read (the key being inserted by another thread) only sends the
-// row to the full probe walk.
+// Code of key k in a finished table, NO_CODE when absent.
 template <int KW>
-__device__ __forceinline__ int64_t d_home(const dtable& t, uint64_t k) {
-    if (KW == 8 && k == D_EMPTY8) return -1;
-    const uint64_t slot = dhash<KW>(k) & t.mask;
-    return t.keys[slot] == k ? (int64_t)slot : -1;
-}
-
-template <int KW>
-__global__ void k_dict_insert(const void* __restrict__ keys, int64_t n, int kind, dtable t, int assign,
-                              unsigned long long* __restrict__ counter) {
-    const int64_t step = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i0 < n; i0 += step * DU) {
-        uint64_t k[DU];
-        int64_t home[DU];
-#pragma unroll
-        for (int q = 0; q < DU; ++q) k[q] = i0 + q * step < n ? dkey<KW>(keys, i0 + q * step, kind) : 0;
-#pragma unroll
-        for (int q = 0; q < DU; ++q) home[q] = i0 + q * step < n ? d_home<KW>(t, k[q]) : 0;
-#pragma unroll
-        for (int q = 0; q < DU; ++q) {
-            if (i0 + q * step >= n || home[q] >= 0) continue;
-            bool ins;
-            int64_t s = d_find<KW>(t, k[q], true, &ins);
-            if (ins) {
-                unsigned long long c = atomicAdd(counter, 1ull);
-                if (assign) t.codes[s] = c;
-            }
+__device__ __forceinline__ uint64_t d_find(const dtable& t, uint64_t k) {
+    if (KW == 8 && k == D_EMPTY) return t.w[2 * (t.mask + 1) + 1];
+    uint64_t slot = dhash<KW>(k) & t.mask;
+    for (uint64_t p = 0, lim = t.mask < GX_PROBE_LIMIT ? t.mask : GX_PROBE_LIMIT - 1; p <= lim; ++p) {
+        if constexpr (KW == 4) {
+            const unsigned long long cur = t.w[slot];
+            if (cur == D_EMPTY) return NO_CODE;
+            if ((uint32_t)(cur >> 32) == (uint32_t)k) return (uint32_t)cur;
+        } else {
+            const ulonglong2 cur = reinterpret_cast<const ulonglong2*>(t.w)[slot];
+            if (cur.x == D_EMPTY) return NO_CODE;
+            if (cur.x == k) return cur.y;
         }
+        slot = (slot + 1) & t.mask;
     }
-}
-
-// Ready dictionary: insert value -> smallest position.
-template <int KW>
-__global__ void k_dict_insert_positions(const void* __restrict__ dict, int64_t n, int kind, dtable t) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        bool ins;
-        int64_t s = d_find<KW>(t, dkey<KW>(dict, i, kind), true, &ins);
-        if (s >= 0) atomicMin(&t.codes[s], (unsigned long long)i);
-    }
+    return NO_CODE;
 }
 
 __device__ __forceinline__ void store_code(void* out, int w, int64_t i, uint64_t c) {
@@ -134,69 +157,140 @@ __device__ __forceinline__ void store_code(void* out, int w, int64_t i, uint64_t
     }
 }
 
+// Rows per thread per round: their keys are loaded, then their home slots
+// read, all at once, so each thread keeps DU independent table reads in
+// flight instead of one dependent chain.
+constexpr int DU = 4;
+constexpr int D_NT = 256;
+
+// Inserts every row's key and writes its code.  Bound by one random L2 sector
+// per row.  Order-preserving codes of 10^8 int32 rows with 2^16 values: 1.44 ms
+// a call (1.81 with a key table and a code table read in two passes).
 template <int KW>
-__global__ void k_dict_lookup(const void* __restrict__ keys, int64_t n, int kind, dtable t, void* out, int ow,
-                              uint64_t missing) {
-    const int64_t step = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i0 < n; i0 += step * DU) {
-        uint64_t k[DU];
-        int64_t slot[DU];
+__global__ void __launch_bounds__(D_NT) k_dict_encode(const void* __restrict__ keys, int64_t n, int kind, dtable t,
+                                                      unsigned long long* __restrict__ counter,
+                                                      void* __restrict__ dkeys, void* __restrict__ out, int ow) {
+    const int64_t step = (int64_t)gridDim.x * D_NT;
+    // Whole warps stay in the loop together: rows that meet a pending code
+    // are tried again after the warp has regrouped.
+    const int64_t rounds = (n + step * DU - 1) / (step * DU);
+    for (int64_t r = 0; r < rounds; ++r) {
+        const int64_t i0 = r * step * DU + blockIdx.x * (int64_t)D_NT + threadIdx.x;
+        uint64_t k[DU], c[DU];
 #pragma unroll
         for (int q = 0; q < DU; ++q) k[q] = i0 + q * step < n ? dkey<KW>(keys, i0 + q * step, kind) : 0;
 #pragma unroll
-        for (int q = 0; q < DU; ++q) slot[q] = i0 + q * step < n ? d_home<KW>(t, k[q]) : 0;
+        for (int q = 0; q < DU; ++q) c[q] = i0 + q * step < n ? d_home<KW>(t, k[q]) : 0;
 #pragma unroll
         for (int q = 0; q < DU; ++q) {
-            if (i0 + q * step >= n || slot[q] >= 0) continue;
-            bool ins;
-            slot[q] = d_find<KW>(t, k[q], false, &ins);
+            if (!__any_sync(0xffffffffu, c[q] == NO_CODE)) continue;
+            if (c[q] == NO_CODE) c[q] = d_insert<KW>(t, k[q], counter, dkeys);
+            for (uint32_t round = 0; __any_sync(0xffffffffu, c[q] == PENDING); ++round) {
+                __syncwarp();
+                if (c[q] != PENDING) continue;
+                if (round < D_WAIT_LIMIT) c[q] = d_insert<KW>(t, k[q], counter, dkeys);
+                else {
+                    atomicExch(t.overflow, 1);
+                    c[q] = NO_CODE;
+                }
+            }
         }
-        uint64_t c[DU];
 #pragma unroll
-        for (int q = 0; q < DU; ++q) c[q] = i0 + q * step < n && slot[q] >= 0 ? t.codes[slot[q]] : NO_CODE;
+        for (int q = 0; q < DU; ++q)
+            if (i0 + q * step < n) store_code(out, ow, i0 + q * step, c[q]);
+    }
+}
+
+// Replaces first-insert codes by ranks: out[i] = rank[code[i]].
+template <typename T>
+__global__ void __launch_bounds__(D_NT) k_dict_remap(const T* codes, int64_t n,
+                                                     const T* __restrict__ rank, void* out, int ow) {
+    const int64_t step = (int64_t)gridDim.x * D_NT;
+    for (int64_t i0 = blockIdx.x * (int64_t)D_NT + threadIdx.x; i0 < n; i0 += step * DU) {
+        T c[DU];
+#pragma unroll
+        for (int q = 0; q < DU; ++q) c[q] = i0 + q * step < n ? codes[i0 + q * step] : T(0);
+#pragma unroll
+        for (int q = 0; q < DU; ++q) c[q] = __ldg(rank + c[q]);
+#pragma unroll
+        for (int q = 0; q < DU; ++q)
+            if (i0 + q * step < n) store_code(out, ow, i0 + q * step, c[q]);
+    }
+}
+template <typename T>
+__global__ void k_dict_rank(const int64_t* __restrict__ sorted_src, int64_t m, T* __restrict__ rank) {
+    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < m; r += (int64_t)gridDim.x * blockDim.x)
+        rank[sorted_src[r]] = (T)r;
+}
+
+// Ready dictionary: insert value -> smallest position.
+template <int KW>
+__global__ void k_dict_insert_positions(const void* __restrict__ dict, int64_t n, int kind, dtable t) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const uint64_t k = dkey<KW>(dict, i, kind);
+        if (KW == 8 && k == D_EMPTY) {
+            atomicMin(t.w + 2 * (t.mask + 1) + 1, (unsigned long long)i);
+            continue;
+        }
+        const unsigned long long word = (unsigned long long)k << 32 | (uint32_t)min(i, (int64_t)PENDING4 - 1);
+        uint64_t slot = dhash<KW>(k) & t.mask;
+        bool done = false;
+        for (uint64_t p = 0, lim = t.mask < GX_PROBE_LIMIT ? t.mask : GX_PROBE_LIMIT - 1; p <= lim && !done; ++p) {
+            if constexpr (KW == 4) {
+                unsigned long long cur = ((volatile unsigned long long*)t.w)[slot];
+                if (cur == D_EMPTY) cur = atomicCAS(&t.w[slot], D_EMPTY, word);
+                if (cur == D_EMPTY) done = true;
+                else if ((uint32_t)(cur >> 32) == (uint32_t)k) {
+                    atomicMin(&t.w[slot], word);  // same key: the smaller position
+                    done = true;
+                }
+            } else {
+                unsigned long long* s = t.w + 2 * slot;
+                unsigned long long cur = *(volatile unsigned long long*)s;
+                if (cur == D_EMPTY) cur = atomicCAS(s, D_EMPTY, (unsigned long long)k);
+                if (cur == D_EMPTY || cur == k) {
+                    atomicMin(s + 1, (unsigned long long)i);
+                    done = true;
+                }
+            }
+            slot = (slot + 1) & t.mask;
+        }
+        if (!done) atomicExch(t.overflow, 1);
+    }
+}
+
+template <int KW>
+__global__ void __launch_bounds__(D_NT) k_dict_lookup(const void* __restrict__ keys, int64_t n, int kind, dtable t,
+                                                      void* __restrict__ out, int ow, uint64_t missing) {
+    const int64_t step = (int64_t)gridDim.x * D_NT;
+    for (int64_t i0 = blockIdx.x * (int64_t)D_NT + threadIdx.x; i0 < n; i0 += step * DU) {
+        uint64_t k[DU], c[DU];
+#pragma unroll
+        for (int q = 0; q < DU; ++q) k[q] = i0 + q * step < n ? dkey<KW>(keys, i0 + q * step, kind) : 0;
+#pragma unroll
+        for (int q = 0; q < DU; ++q) c[q] = i0 + q * step < n ? d_home<KW>(t, k[q]) : 0;
+#pragma unroll
+        for (int q = 0; q < DU; ++q)
+            if (c[q] == NO_CODE) c[q] = d_find<KW>(t, k[q]);
 #pragma unroll
         for (int q = 0; q < DU; ++q)
             if (i0 + q * step < n) store_code(out, ow, i0 + q * step, c[q] == NO_CODE ? missing : c[q]);
     }
 }
 
-// Compact occupied slots' keys (for the order-preserving path).
-__global__ void k_dict_compact(dtable t, uint64_t empty, int kw, void* out_keys, unsigned long long* counter,
-                               int64_t* out_slots) {
-    int64_t cap = (int64_t)t.mask + 1;
-    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s <= cap; s += (int64_t)gridDim.x * blockDim.x) {
-        unsigned long long k = t.keys[s];
-        bool live = s < cap ? k != empty : k == empty;
-        if (!live) continue;
-        unsigned long long p = atomicAdd(counter, 1ull);
-        if (kw == 4) static_cast<unsigned*>(out_keys)[p] = (unsigned)k;
-        else static_cast<unsigned long long*>(out_keys)[p] = k;
-        out_slots[p] = s;
-    }
-}
-__global__ void k_dict_rank(const int64_t* __restrict__ sorted_src, const int64_t* __restrict__ slots, int64_t m,
-                            dtable t) {
-    for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < m; r += (int64_t)gridDim.x * blockDim.x)
-        t.codes[slots[sorted_src[r]]] = (unsigned long long)r;
-}
-
 struct table_bufs {
-    dbuf keys, codes, flags;
+    dbuf slots, flags;  // flags: overflow, then the code counter
     dtable t;
 };
 
 table_bufs make_table(int64_t cap, int kw, cudaStream_t s) {
     table_bufs b;
-    b.keys = dbuf((size_t)(cap + 1) * 8, s);
-    b.codes = dbuf((size_t)(cap + 1) * 8, s);
+    const size_t bytes = (size_t)(cap + 1) * (kw == 4 ? 8 : 16);
+    b.slots = dbuf(bytes, s);
     b.flags = dbuf(16, s);
-    uint64_t empty = kw == 4 ? D_EMPTY4 : D_EMPTY8;
-    fill_u64(b.keys.get(), empty, cap, s);
-    fill_u64(b.keys.get<char>() + cap * 8, empty ^ 1ull, 1, s);  // sentinel slot starts unused
-    fill_u64(b.codes.get(), NO_CODE, cap + 1, s);
+    GX_CUDA(cudaMemsetAsync(b.slots.get(), 0xFF, bytes, s));
     GX_CUDA(cudaMemsetAsync(b.flags.get(), 0, 16, s));
-    b.t.keys = b.keys.get<unsigned long long>();
-    b.t.codes = b.codes.get<unsigned long long>();
+    b.t.w = b.slots.get<unsigned long long>();
     b.t.mask = (uint64_t)cap - 1;
     b.t.overflow = b.flags.get<int>();
     return b;
@@ -242,14 +336,25 @@ void dictionary_encode(const gx_column_view& v, int encode_type, int64_t size_hi
     const int ow = size_of(encode_type);
     owned_col res = make_col(encode_type, c.n, s);
     int64_t cap = table_capacity(c, size_hint, load_factor, s);
+    // Order-preserving codes start as first-insert codes, in the result itself
+    // when it is wide enough.
+    dbuf narrow;
+    void* first = res.buf.get();
+    const int fw = mode == 1 && ow < 4 ? 4 : ow;
+    if (fw != ow) {
+        narrow = dbuf((size_t)c.n * fw, s);
+        first = narrow.get();
+    }
     for (int attempt = 0; attempt < 6; ++attempt, cap *= 4) {
         table_bufs tb = make_table(cap, kw, s);
         unsigned long long* counter = reinterpret_cast<unsigned long long*>(tb.flags.get<char>() + 8);
-        int g = grid_for(c.n, 256, 8);
+        dbuf dk;  // distinct keys in code order
+        if (mode == 1) dk = dbuf((size_t)std::min<int64_t>(cap + 1, std::max<int64_t>(c.n, 1)) * kw, s);
+        int g = grid_for(c.n, D_NT, 8);
         if (c.n > 0) {
             GX_PROF("dict_insert", s);
-            if (kw == 4) k_dict_insert<4><<<g, 256, 0, s>>>(c.data, c.n, kind, tb.t, mode == 0, counter);
-            else k_dict_insert<8><<<g, 256, 0, s>>>(c.data, c.n, kind, tb.t, mode == 0, counter);
+            if (kw == 4) k_dict_encode<4><<<g, D_NT, 0, s>>>(c.data, c.n, kind, tb.t, counter, dk.get(), first, fw);
+            else k_dict_encode<8><<<g, D_NT, 0, s>>>(c.data, c.n, kind, tb.t, counter, dk.get(), first, fw);
             GX_LAUNCHED();
         }
         int hflags[4];
@@ -260,29 +365,29 @@ void dictionary_encode(const gx_column_view& v, int encode_type, int64_t size_hi
         std::memcpy(&ndv_u, &hflags[2], 8);
         int64_t ndv = (int64_t)ndv_u;
         if (mode == 1 && ndv > 0) {
-            dbuf dk((size_t)ndv * kw, s), dslot((size_t)ndv * 8, s), cnt(8, s);
-            GX_CUDA(cudaMemsetAsync(cnt.get(), 0, 8, s));
-            uint64_t empty = kw == 4 ? D_EMPTY4 : D_EMPTY8;
-            k_dict_compact<<<grid_for(cap + 1, 256, 8), 256, 0, s>>>(tb.t, empty, kw, dk.get(), cnt.get<unsigned long long>(),
-                                                                   dslot.get<int64_t>());
-            GX_LAUNCHED();
-            // Sort distinct keys (with their compaction index) in value order.
+            // Sort the distinct keys (with their codes) in value order.
             col kc;
             kc.data = dk.get();
             kc.n = ndv;
             kc.type = c.type;
-            dbuf sk((size_t)ndv * kw, s), si((size_t)ndv * 8, s);
+            dbuf sk((size_t)ndv * kw, s), si((size_t)ndv * 8, s), rank((size_t)ndv * fw, s);
             radix_sort(kc, nullptr, 8, true, 0, -1, false, sk.get(), si.get(), nullptr, 0, s);
-            k_dict_rank<<<grid_for(ndv, 256, 8), 256, 0, s>>>(si.get<int64_t>(), dslot.get<int64_t>(), ndv, tb.t);
-            GX_LAUNCHED();
-        }
-        if (c.n > 0) {
+            const int rg = grid_for(ndv, 256, 8);
             GX_PROF("dict_lookup", s);
-            if (kw == 4) k_dict_lookup<4><<<g, 256, 0, s>>>(c.data, c.n, kind, tb.t, res.buf.get(), ow, 0);
-            else k_dict_lookup<8><<<g, 256, 0, s>>>(c.data, c.n, kind, tb.t, res.buf.get(), ow, 0);
+            if (fw == 8) {
+                k_dict_rank<<<rg, 256, 0, s>>>(si.get<int64_t>(), ndv, rank.get<unsigned long long>());
+                GX_LAUNCHED();
+                k_dict_remap<<<g, D_NT, 0, s>>>(static_cast<const unsigned long long*>(first), c.n,
+                                               rank.get<unsigned long long>(), res.buf.get(), ow);
+            } else {
+                k_dict_rank<<<rg, 256, 0, s>>>(si.get<int64_t>(), ndv, rank.get<unsigned>());
+                GX_LAUNCHED();
+                k_dict_remap<<<g, D_NT, 0, s>>>(static_cast<const unsigned*>(first), c.n, rank.get<unsigned>(),
+                                               res.buf.get(), ow);
+            }
             GX_LAUNCHED();
+            GX_CUDA(cudaStreamSynchronize(s));
         }
-        GX_CUDA(cudaStreamSynchronize(s));
         *dict_size = ndv;
         *out = to_gx_column(std::move(res));
         return;
@@ -314,10 +419,10 @@ void dictionary_encode_with_dict(const gx_column_view& v, const gx_column_view& 
         int ovf = read_scalar(tb.flags.get<int>(), s);
         if (ovf) continue;
         if (c.n > 0) {
-            int g = grid_for(c.n, 256, 8);
+            int g = grid_for(c.n, D_NT, 8);
             uint64_t missing = (uint64_t)(uint32_t)0x80000000u;
-            if (kw == 4) k_dict_lookup<4><<<g, 256, 0, s>>>(c.data, c.n, kind, tb.t, res.buf.get(), 4, missing);
-            else k_dict_lookup<8><<<g, 256, 0, s>>>(c.data, c.n, kind, tb.t, res.buf.get(), 4, missing);
+            if (kw == 4) k_dict_lookup<4><<<g, D_NT, 0, s>>>(c.data, c.n, kind, tb.t, res.buf.get(), 4, missing);
+            else k_dict_lookup<8><<<g, D_NT, 0, s>>>(c.data, c.n, kind, tb.t, res.buf.get(), 4, missing);
             GX_LAUNCHED();
         }
         GX_CUDA(cudaStreamSynchronize(s));

@@ -387,3 +387,39 @@ def test_join_hash_and_partition_hints_give_the_sort_result(algo, mat):
     got = np.lexsort((cols[2], cols[1]))
     el, er = O.join_pairs(lk, rk)
     assert np.array_equal(cols[1][got], el) and np.array_equal(cols[2][got], er)
+
+
+@pytest.mark.parametrize("kdt", [np.int32, np.float32, np.int64, np.float64, np.int16])
+@pytest.mark.parametrize("enc,edt", [(gx.INT32, np.int32), (gx.INT64, np.int64), (gx.UINT8, np.uint8)])
+def test_dictionary_side_by_side_slots_and_remap(kdt, enc, edt):
+    # Keys whose bits are all ones (an empty slot's marker), the lowest key,
+    # zeros of both signs, and every width of the codes: hash codes are a dense
+    # bijection, ordered codes the ranks, ready codes the smallest positions.
+    ndv, n = 200, 70_003
+    rng = np.random.default_rng(11)
+    if np.dtype(kdt).kind == "f":
+        vals = np.unique((rng.integers(-400, 400, 4 * ndv) / 4).astype(kdt))[:ndv]
+    else:
+        lim = np.iinfo(kdt)
+        vals = np.unique(np.concatenate([[-1, lim.min, lim.max, 0], rng.integers(lim.min, lim.max, 4 * ndv)]))
+        vals = vals.astype(kdt)[: ndv - 2]
+        vals = np.unique(np.concatenate([vals, np.array([-1, lim.max], kdt)]))
+    col = vals[rng.integers(0, len(vals), n)]
+    col[: len(vals)] = vals
+    if np.dtype(kdt).kind == "f":
+        col[col == 0] = np.where(rng.integers(0, 2, int((col == 0).sum())) == 1, 0.0, -0.0)
+    d = to_dev(col)
+    rank = np.searchsorted(vals, col)
+    codes, m = gx.dictionary_encode(d, enc, ordered=True)
+    assert m == len(vals) and np.array_equal(codes.cpu().numpy(), rank.astype(edt))
+    codes, m = gx.dictionary_encode(d, enc)
+    c = codes.cpu().numpy()
+    assert m == len(vals) and len(np.unique(c)) == m and c.max() == m - 1
+    assert len(np.unique(np.stack([c.astype(np.int64), rank], 1), axis=0)) == m
+    if enc == gx.INT32:
+        half = np.concatenate([vals[::2], vals[::-2], vals[::2]])  # duplicated values, some absent
+        got = gx.dictionary_encode_with_dict(d, to_dev(half)).cpu().numpy()
+        first = {}
+        for i, v in enumerate(half):
+            first.setdefault(float(v) + 0.0, i)
+        assert np.array_equal(got, np.array([first.get(float(v) + 0.0, -2**31) for v in col], np.int32))
