@@ -134,6 +134,9 @@ constexpr int HGB_UNROLL = 4;
 // dense-id kernel (7 aggregates at 2^28 rows, 2^16 groups: 2.52 ms against
 // 2.60 with two and 2.98 with four).
 constexpr int HU_UNROLL = 3;
+// The dense-id kernel on small units: CTAs of this many threads, several per
+// SM (see hash_units_aggregate).
+constexpr int HU_SMALL_NT = 256;
 
 template <int KW, bool SMEM, int NV, class... ACCS>
 __global__ void __launch_bounds__(HGB_NT, 1) k_hash_groupby(const void* __restrict__ keys, int64_t n,
@@ -651,8 +654,8 @@ __device__ __forceinline__ uint64_t ud_load_key(const void* keys, int64_t i, int
     return canon64(__ldg(static_cast<const unsigned long long*>(keys) + i), kind);
 }
 
-template <int KW, int NV, class... ACCS>
-__global__ void __launch_bounds__(HGB_NT, 1) k_units_dense(const void* __restrict__ keys, int key_kind, agg_desc d,
+template <int NT, int KW, int NV, class... ACCS>
+__global__ void __launch_bounds__(NT, NT == HGB_NT ? 1 : 4) k_units_dense(const void* __restrict__ keys, int key_kind, agg_desc d,
                                                             const part_unit* __restrict__ units,
                                                             const int64_t* __restrict__ n_units, uint32_t s_slots,
                                                             uint32_t gcap, int reps, uint32_t gpp, int shift,
@@ -664,7 +667,7 @@ __global__ void __launch_bounds__(HGB_NT, 1) k_units_dense(const void* __restric
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_fill, s_spill;
     __shared__ unsigned long long s_base;
-    __shared__ uint32_t s_q[HGB_NT / 32][31 + 32 * HU_UNROLL];
+    __shared__ uint32_t s_q[NT / 32][31 + 32 * HU_UNROLL];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
     const int NA = CP ? (int)sizeof...(ACCS) : d.n_acc;
@@ -710,18 +713,18 @@ __global__ void __launch_bounds__(HGB_NT, 1) k_units_dense(const void* __restric
         const int rep = (int)(threadIdx.x & (unsigned)(R - 1));
         unsigned* my_counts = counts + rep;
         uint64_t* my_acc = acc + rep;
-        for (uint32_t i = threadIdx.x; i < s_slots; i += HGB_NT) t.slots[i] = UD_EMPTY;
+        for (uint32_t i = threadIdx.x; i < s_slots; i += NT) t.slots[i] = UD_EMPTY;
         if (KW == 8)
-            for (uint32_t i = threadIdx.x; i < gcap; i += HGB_NT) t.gkey[i] = (kt)UD_UNSET;
-        for (uint32_t i = threadIdx.x; i < GRu; i += HGB_NT) counts[i] = 0;
+            for (uint32_t i = threadIdx.x; i < gcap; i += NT) t.gkey[i] = (kt)UD_UNSET;
+        for (uint32_t i = threadIdx.x; i < GRu; i += NT) counts[i] = 0;
         for (int a = 0; a < NA; ++a) {
             const uint64_t idv = dev_::acc_ident(d.acc_op[a], d.acc_kind[a]);
             uint64_t* base = acc + (size_t)a * GR;
-            for (uint32_t i = threadIdx.x; i < GRu; i += HGB_NT) base[i] = idv;
+            for (uint32_t i = threadIdx.x; i < GRu; i += NT) base[i] = idv;
         }
         if (threadIdx.x == 0) { s_fill = 0; s_spill = 0; }
         __syncthreads();
-        const int64_t tile = (int64_t)HGB_NT * HU_UNROLL;
+        const int64_t tile = (int64_t)NT * HU_UNROLL;
         auto drain = [&](uint32_t off, bool live) {
             const int64_t i = un.begin + off;
             kt kq = 0;
@@ -749,7 +752,7 @@ __global__ void __launch_bounds__(HGB_NT, 1) k_units_dense(const void* __restric
             uint64_t v[HU_UNROLL][NV];
 #pragma unroll
             for (int q = 0; q < HU_UNROLL; ++q) {
-                const int64_t i = base + q * HGB_NT + threadIdx.x;
+                const int64_t i = base + q * NT + threadIdx.x;
                 if (i < un.end) {
                     kw[q] = (kt)ud_load_key<KW>(keys, i, key_kind);
                     load_vals(i, v[q]);
@@ -760,7 +763,7 @@ __global__ void __launch_bounds__(HGB_NT, 1) k_units_dense(const void* __restric
             uint32_t gid[HU_UNROLL];
 #pragma unroll
             for (int q = 0; q < HU_UNROLL; ++q) {
-                const bool valid = base + q * HGB_NT + threadIdx.x < un.end;
+                const bool valid = base + q * NT + threadIdx.x < un.end;
                 gid[q] = 0xFFFFFFFFu;
                 if (valid) {
                     const uint32_t h = key_hash<KW>(kw[q]);
@@ -774,7 +777,7 @@ __global__ void __launch_bounds__(HGB_NT, 1) k_units_dense(const void* __restric
             }
 #pragma unroll
             for (int q = 0; q < HU_UNROLL; ++q) {
-                const int64_t i = base + q * HGB_NT + threadIdx.x;
+                const int64_t i = base + q * NT + threadIdx.x;
                 const bool valid = i < un.end;
                 const bool hit = valid && gid[q] < gcap;
                 const bool miss = valid && !hit;
@@ -807,7 +810,7 @@ __global__ void __launch_bounds__(HGB_NT, 1) k_units_dense(const void* __restric
         const bool append = final_groups && (int64_t)(s_base + ng) <= rec_cap;
         if (append || !final_groups) {
             // Ids are dense: group j of the unit is record s_base + j.
-            for (uint32_t j = threadIdx.x; j < ng; j += HGB_NT) {
+            for (uint32_t j = threadIdx.x; j < ng; j += NT) {
                 const uint64_t kwv = (uint64_t)t.gkey[j];
                 unsigned long long c = 0;
                 int first = -1;
@@ -968,6 +971,7 @@ struct units_args {
     unsigned long long* ocount;
     int64_t rec_cap;
     int* rec_ovf;
+    bool small;  // dense-id kernel: CTAs of HU_SMALL_NT threads
 };
 
 template <int KW, int NV, class... ACCS>
@@ -985,15 +989,22 @@ static bool try_units_spec(int grid, size_t smem, cudaStream_t s, const agg_desc
     return true;
 }
 
+template <int NT, int KW, int NV, class... ACCS>
+static void launch_units_dense_nt(int grid, size_t smem, cudaStream_t s, const agg_desc& d, const units_args& a,
+                                  uint32_t gcap, uint32_t gpp) {
+    GX_CUDA(cudaFuncSetAttribute(k_units_dense<NT, KW, NV, ACCS...>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)smem));
+    k_units_dense<NT, KW, NV, ACCS...><<<grid, NT, smem, s>>>(a.keys, a.kind, d, a.units, a.n_units, a.slots, gcap,
+                                                              a.reps, gpp, a.shift, a.g, a.orec, a.ocount,
+                                                              a.rec_cap, a.rec_ovf);
+}
+
 template <int KW, int NV, class... ACCS>
 static bool launch_units_dense(int grid, size_t smem, cudaStream_t s, const agg_desc& d, const units_args& a,
                                uint32_t gcap, uint32_t gpp) {
     GX_PROF("partition_aggregate", s);
-    GX_CUDA(cudaFuncSetAttribute(k_units_dense<KW, NV, ACCS...>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem));
-    k_units_dense<KW, NV, ACCS...><<<grid, HGB_NT, smem, s>>>(a.keys, a.kind, d, a.units, a.n_units, a.slots, gcap,
-                                                              a.reps, gpp, a.shift, a.g, a.orec, a.ocount,
-                                                              a.rec_cap, a.rec_ovf);
+    if (a.small) launch_units_dense_nt<HU_SMALL_NT, KW, NV, ACCS...>(grid, smem, s, d, a, gcap, gpp);
+    else launch_units_dense_nt<HGB_NT, KW, NV, ACCS...>(grid, smem, s, d, a, gcap, gpp);
     return true;
 }
 
@@ -1168,7 +1179,7 @@ void hash_groupby(const col& key_in, const agg_plan& p, gx_groupby_hint* hint, c
 bool hash_units_aggregate(const void* keys, int kw, int kind, const agg_desc& d, const part_unit* units,
                           const int64_t* n_units, int64_t gpp, int shift, uint64_t* grec, uint64_t gcap, int* gflags,
                           uint64_t* orec, unsigned long long* ocount, int64_t rec_cap, int* rec_ovf, cudaStream_t s,
-                          bool dense_only) {
+                          bool dense_only, int64_t unit_rows) {
     const size_t budget = 200 * 1024;
     const size_t per_rep = 4 + 8 * (size_t)d.n_acc;
     // Slots for the fullest partition expected (Poisson tail), at load <= 1/4:
@@ -1190,14 +1201,26 @@ bool hash_units_aggregate(const void* keys, int kw, int kind, const agg_desc& d,
         };
         // Slots at load <= 1/4, else <= 1/2 (e.g. ~2K groups with 7 aggregates).
         if (need(1) > budget) dslots = (uint32_t)next_pow2((uint64_t)std::max(64.0, 2.0 * gmax));
+        // Small units (many partitions of few rows): four 256-thread CTAs per
+        // SM instead of one of 1024, so that one unit's table set-up, barriers
+        // and merge overlap another's rows.  2^26 rows, 7 aggregates, int32
+        // keys, ms per call with large / small CTAs: 1024 rows per partition
+        // 5.82 / 3.96, 4096: 3.34 / 2.64, 16384: 2.47 / 2.24, 65536: 2.82 /
+        // 2.62, 262144: 1.68 / 1.62 (SUM + COUNT of int64 keys 1.31 / 1.36).
+        // With fewer units than CTAs large ones win (2^18 rows in 16
+        // partitions: 0.17 / 0.20), so the caller passes unit_rows = 0 there.
+        constexpr size_t SMALL_BUDGET = 50 * 1024;
+        const bool small = unit_rows > 0 && unit_rows < (1 << 17) && need(1) <= SMALL_BUDGET;
+        const size_t room = small ? SMALL_BUDGET : budget;
         size_t r = 16;
-        while (r > 1 && need(r) > budget) r >>= 1;
-        if (need(r) <= budget) {
+        while (r > 1 && need(r) > room) r >>= 1;
+        if (need(r) <= room) {
             const units_args a{keys, kind, units, n_units, dslots, (int)r, shift,
-                               gtable{grec, gcap - 1, gflags, gflags + 1}, orec, ocount, rec_cap, rec_ovf};
+                               gtable{grec, gcap - 1, gflags, gflags + 1}, orec, ocount, rec_cap, rec_ovf, small};
             const uint32_t g32 = (uint32_t)std::min<int64_t>(std::max<int64_t>(gpp, 1), ids);
-            if (kw == 4 ? units_dense_dispatch<4>(grid, need(r), s, d, a, ids, g32)
-                        : units_dense_dispatch<8>(grid, need(r), s, d, a, ids, g32)) {
+            const int dgrid = small ? grid * 4 : grid;
+            if (kw == 4 ? units_dense_dispatch<4>(dgrid, need(r), s, d, a, ids, g32)
+                        : units_dense_dispatch<8>(dgrid, need(r), s, d, a, ids, g32)) {
                 GX_LAUNCHED();
                 return true;
             }
@@ -1215,7 +1238,7 @@ bool hash_units_aggregate(const void* keys, int kw, int kind, const agg_desc& d,
     const size_t smem = (((size_t)slots * kw + 15) & ~size_t(15)) + (((size_t)slots * 4 * reps + 15) & ~size_t(15)) +
                         (size_t)slots * reps * 8 * d.n_acc;
     units_args a{keys, kind, units, n_units, slots, (int)reps, shift,
-                 gtable{grec, gcap - 1, gflags, gflags + 1}, orec, ocount, rec_cap, rec_ovf};
+                 gtable{grec, gcap - 1, gflags, gflags + 1}, orec, ocount, rec_cap, rec_ovf, false};
     GX_PROF("partition_aggregate", s);
     if (kw == 4) units_dispatch<4>(grid, smem, s, d, a);
     else units_dispatch<8>(grid, smem, s, d, a);

@@ -269,9 +269,15 @@ __global__ void __launch_bounds__(PS_NT, 2) k_part_scatter_r(const void* __restr
 // + gridDim.x, ...), with each tile's column slices brought into shared
 // memory by the copy engine (cp.async.bulk on an mbarrier) one tile ahead, so
 // the loads of tile t+1 overlap the ranking and writes of tile t and no
-// column value occupies a register.  STABLE ranks a tile as k_part_scatter
-// does (digit, then row order); otherwise each row's rank within its digit
-// is one shared atomic (any order inside a (digit, tile) run).  Each output
+// column value occupies a register.  Each row's rank within its digit is one
+// shared atomic (any order inside a (digit, tile) run).  SECOND, the second
+// pass of a two-pass partition, has to keep the rows of each earlier digit
+// together and in that digit's order: its input is ordered by the earlier
+// digit, so a tile nearly always lies within one value of it and any order
+// does; a tile that spans several values ranks them one after the other, a
+// barrier apart.  (Ranking every row in input order by __match_any_sync took
+// 1.8 ms per 2^28 rows alone, and its per-warp counts left no room for three
+// 8-byte columns.)  Each output
 // position j then reads its source row from the shared copy and writes every
 // column to gbase[digit] + j.  Used when every loaded column starts on a
 // 16-byte boundary and two tiles of the columns fit in shared memory.
@@ -284,12 +290,10 @@ constexpr uint32_t PB_WAIT_LIMIT = 1u << 22;
 struct pb_layout {
     uint32_t in_off[MAX_VCOLS + 2];  // column c's slice within one stage
     uint32_t stage_bytes;            // one tile of every loaded column
-    uint32_t whist, qsum, pk, gbase, dbase, total;
+    uint32_t pk, gbase, dbase, total;
 };
 
-// Shared-memory layout; the per-warp counts of the stable ranking are only
-// laid out when `stable`.
-__host__ __device__ inline pb_layout pb_make_layout(const move_cols& mc, bool stable) {
+__host__ __device__ inline pb_layout pb_make_layout(const move_cols& mc) {
     pb_layout L{};
     uint32_t o = 0;
     for (int c = 0; c < mc.n; ++c) {
@@ -298,8 +302,6 @@ __host__ __device__ inline pb_layout pb_make_layout(const move_cols& mc, bool st
     }
     L.stage_bytes = o;
     o *= 2;
-    L.whist = o; if (stable) o += PB_WARPS * PS_BINS * 2;   // u16 per-warp digit counts
-    L.qsum = o;  if (stable) o += 4 * PS_BINS * 2;          // u16 sums over 8-warp quarters
     L.pk = o;    o += PS_TILE * 4;              // u32 per staged position: source row | digit << 16
     L.gbase = o; o += PS_BINS * 8;              // int64 output base per digit
     L.dbase = o; o += PS_BINS * 4;              // u32 first staged position per digit
@@ -307,7 +309,7 @@ __host__ __device__ inline pb_layout pb_make_layout(const move_cols& mc, bool st
     return L;
 }
 
-template <int KW, int NC, bool STABLE>
+template <int KW, int NC, bool SECOND>
 __global__ void __launch_bounds__(PB_NT, 1) k_part_scatter_bulk(const void* __restrict__ keys, int64_t n, int kind,
                                                                 int shift, int dbits, int64_t ntiles,
                                                                 const int64_t* __restrict__ offsets, move_cols mc,
@@ -315,10 +317,8 @@ __global__ void __launch_bounds__(PB_NT, 1) k_part_scatter_bulk(const void* __re
     extern __shared__ __align__(128) unsigned char pb_smem[];
     __shared__ __align__(8) unsigned long long bars[2];
     __shared__ unsigned wsum[PS_BINS / 32];
-    __shared__ unsigned thist[PS_BINS];  // unstable ranking: running count per digit
+    __shared__ unsigned thist[PS_BINS];  // running count per digit
     __shared__ int s_err;
-    unsigned short* whist = reinterpret_cast<unsigned short*>(pb_smem + L.whist);
-    unsigned short* qsum = reinterpret_cast<unsigned short*>(pb_smem + L.qsum);
     unsigned* pk = reinterpret_cast<unsigned*>(pb_smem + L.pk);
     int64_t* gbase = reinterpret_cast<int64_t*>(pb_smem + L.gbase);
     unsigned* dbase = reinterpret_cast<unsigned*>(pb_smem + L.dbase);
@@ -342,13 +342,13 @@ __global__ void __launch_bounds__(PB_NT, 1) k_part_scatter_bulk(const void* __re
     };
     auto full = [&](int64_t tile) { return (tile + 1) * (int64_t)PS_TILE <= n; };
     unsigned char* stage = nullptr;
-    // Digit of the tile's row `local` (key column of the current stage).
-    auto digit_at = [&](int local) -> unsigned {
+    // Partition hash of the tile's row `local` (key column of the current stage).
+    auto hash_at = [&](int local) -> unsigned {
         uint64_t kb;
         if (KW == 4) kb = reinterpret_cast<const unsigned*>(stage + L.in_off[0])[local];
         else kb = reinterpret_cast<const unsigned long long*>(stage + L.in_off[0])[local];
         kb = KW == 4 ? canon32((uint32_t)kb, kind) : canon64(kb, kind);
-        return (part_hash<KW>(kb) >> shift) & (bins - 1);
+        return part_hash<KW>(kb);
     };
     if (t == 0) {
         dev_::mbar_init(bar0, 1);
@@ -368,7 +368,6 @@ __global__ void __launch_bounds__(PB_NT, 1) k_part_scatter_bulk(const void* __re
             if (tile < ntiles && full(tile)) { issue(tile, b); pending |= 1u << b; }
         }
     }
-    const unsigned lt = (1u << lane) - 1u;
     int it = 0;
     for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++it) {
         const int b = it & 1;
@@ -400,62 +399,49 @@ __global__ void __launch_bounds__(PB_NT, 1) k_part_scatter_bulk(const void* __re
             }
             __syncthreads();
         }
-        // Rank the tile's rows within their digit.  STABLE (every pass after
-        // the first of a multi-pass partition, which LSD order needs): per-warp
-        // counts over rows warp*128 + k*32 + lane, then a cross-warp prefix.
-        // Otherwise one shared atomic per row gives an arbitrary order within
-        // each (digit, tile) run, which a single-pass partition allows.
+        // Rank the tile's rows within their digit.
         unsigned dig[PB_IPT], rank[PB_IPT];
         unsigned tot = 0, incl = 0;
-        if constexpr (STABLE) {
-            for (int i = lane; i < PS_BINS; i += 32) whist[warp * PS_BINS + i] = 0;
-            __syncwarp();
-#pragma unroll
-            for (int k = 0; k < PB_IPT; ++k) {
-                const int local = warp * 32 * PB_IPT + k * 32 + lane;
-                const bool valid = local < tile_n;
-                const unsigned d = valid ? digit_at(local) : 0xFFFFu;
-                dig[k] = d;
-                const unsigned peers = __match_any_sync(0xffffffffu, d);
-                const unsigned r = __popc(peers & lt);
-                const unsigned prior = valid ? whist[warp * PS_BINS + d] : 0;
-                rank[k] = prior + r;
-                __syncwarp();
-                if (valid && r == 0) whist[warp * PS_BINS + d] = (unsigned short)(prior + __popc(peers));
-                __syncwarp();
-            }
+        unsigned low = 0, high = 0;  // earlier digits (the hash bits below `shift`) of the tile
+        if constexpr (SECOND) {
+            // The same `low` and `high` in every thread (they decide barriers):
+            // every thread's wait has ended, and none timed out.
             __syncthreads();
             if (s_err) break;
-            // Cross-warp exclusive prefix per digit: thread (q, bin) sums warps 8q..8q+7.
-            const int bq = t & (PS_BINS - 1), q = t >> 8;
-            unsigned v[8], s = 0;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) { v[j] = whist[(q * 8 + j) * PS_BINS + bq]; s += v[j]; }
-            qsum[q * PS_BINS + bq] = (unsigned short)s;
-            __syncthreads();
-            unsigned run = 0;
-#pragma unroll
-            for (int qq = 0; qq < 4; ++qq) {
-                const unsigned x = qsum[qq * PS_BINS + bq];
-                if (qq < q) run += x;
-                tot += x;
-            }
-#pragma unroll
-            for (int j = 0; j < 8; ++j) { whist[(q * 8 + j) * PS_BINS + bq] = (unsigned short)run; run += v[j]; }
-        } else {
+            low = hash_at(0) & ((1u << shift) - 1u);
+            high = hash_at(tile_n - 1) & ((1u << shift) - 1u);
+        }
+        if (!SECOND || low == high) {
 #pragma unroll
             for (int k = 0; k < PB_IPT; ++k) {
                 const int local = warp * 32 * PB_IPT + k * 32 + lane;
                 const bool valid = local < tile_n;
-                dig[k] = valid ? digit_at(local) : 0u;
+                dig[k] = valid ? (hash_at(local) >> shift) & (bins - 1) : 0u;
                 rank[k] = valid ? atomicAdd(&thist[dig[k]], 1u) : 0u;
             }
             __syncthreads();
-            if (s_err) break;
-            if (t < PS_BINS) {
-                tot = thist[t];
-                thist[t] = 0;  // ready for the next tile
+        } else {
+            unsigned early[PB_IPT];
+#pragma unroll
+            for (int k = 0; k < PB_IPT; ++k) {
+                const int local = warp * 32 * PB_IPT + k * 32 + lane;
+                const unsigned h = local < tile_n ? hash_at(local) : 0u;
+                dig[k] = (h >> shift) & (bins - 1);
+                rank[k] = 0;
+                early[k] = local < tile_n ? h & ((1u << shift) - 1u) : ~0u;
             }
+            for (unsigned v = low; v <= high; ++v) {
+#pragma unroll
+                for (int k = 0; k < PB_IPT; ++k)
+                    if (early[k] == v) rank[k] = atomicAdd(&thist[dig[k]], 1u);
+                __syncthreads();
+            }
+            __syncthreads();
+        }
+        if (s_err) break;
+        if (t < PS_BINS) {
+            tot = thist[t];
+            thist[t] = 0;  // ready for the next tile
         }
         if (t < PS_BINS) {
             incl = dev_::warp_inclusive_sum(tot);
@@ -473,7 +459,7 @@ __global__ void __launch_bounds__(PB_NT, 1) k_part_scatter_bulk(const void* __re
         for (int k = 0; k < PB_IPT; ++k) {
             const int local = warp * 32 * PB_IPT + k * 32 + lane;
             if (local < tile_n) {
-                const unsigned pos = dbase[dig[k]] + (STABLE ? (unsigned)whist[warp * PS_BINS + dig[k]] : 0u) + rank[k];
+                const unsigned pos = dbase[dig[k]] + rank[k];
                 pk[pos] = (unsigned)local | (dig[k] << 16);
             }
         }
@@ -798,7 +784,7 @@ namespace {
 
 // The bulk-copy scatter applies to 1..4 moved columns when every loaded
 // column is 4 or 8 bytes wide and 16-byte aligned, and two tiles of them fit
-// in shared memory (four columns: up to 24 B per row, single-pass ranking).
+// in shared memory (up to 24 B per row).
 static bool bulk_scatter_ok(const move_cols& mc, const pb_layout& L) {
     if (mc.n < 1 || mc.n > 4) return false;
     for (int c = 0; c < mc.n; ++c) {
@@ -811,13 +797,13 @@ static bool bulk_scatter_ok(const move_cols& mc, const pb_layout& L) {
 
 template <int KW>
 void part_pass(const void* kin, int64_t n, int kind, int shift, int dbits, move_cols& mc, int64_t* counts,
-               int64_t* offs, int* err, bool stable, cudaStream_t s) {
+               int64_t* offs, int* err, bool second, cudaStream_t s) {
     int64_t ntiles = ceil_div(n, PS_TILE);
     const int hist_grid = (int)std::min<int64_t>(ceil_div(ntiles, PH_WARPS), (int64_t)dev().sm_count * 8);
     k_part_hist<KW><<<hist_grid, PH_NT, 0, s>>>(kin, n, kind, shift, dbits, ntiles, counts);
     GX_LAUNCHED();
     exclusive_scan_i64(counts, offs, ((int64_t)1 << dbits) * ntiles, s);
-    const pb_layout L = pb_make_layout(mc, stable);
+    const pb_layout L = pb_make_layout(mc);
     if (mc.n >= 2 && !getenv("GX_PART_NO_BULK") && bulk_scatter_ok(mc, L)) {
         static per_device_flag battr;
         battr.once([] {
@@ -834,11 +820,11 @@ void part_pass(const void* kin, int64_t n, int kind, int shift, int dbits, move_
 #define GX_PB_LAUNCH(NCV, ST)                                                                                       \
     k_part_scatter_bulk<KW, NCV, ST><<<grid, PB_NT, L.total, s>>>(kin, n, kind, shift, dbits, ntiles, \
                                                                           offs, mc, L, err)
-        if (mc.n == 2 && stable) GX_PB_LAUNCH(2, true);
+        if (mc.n == 2 && second) GX_PB_LAUNCH(2, true);
         else if (mc.n == 2) GX_PB_LAUNCH(2, false);
-        else if (mc.n == 3 && stable) GX_PB_LAUNCH(3, true);
+        else if (mc.n == 3 && second) GX_PB_LAUNCH(3, true);
         else if (mc.n == 3) GX_PB_LAUNCH(3, false);
-        else if (stable) GX_PB_LAUNCH(4, true);
+        else if (second) GX_PB_LAUNCH(4, true);
         else GX_PB_LAUNCH(4, false);
 #undef GX_PB_LAUNCH
         GX_LAUNCHED();
@@ -944,10 +930,10 @@ void partition_groupby(const col& key_in, const agg_plan& p, gx_groupby_hint* hi
                 for (int c = 0; c < mc.n; ++c) { m.in[c] = bufs_b[c]; m.iota[c] = 0; m.out[c] = bufs_a[c]; }
             }
             const void* kin = m.in[0];
-            // Only the first digit pass may leave rows unordered within a run.
-            const bool stable = ps > 0;
-            if (kw == 4) part_pass<4>(kin, n, kind, shift, dbits, m, counts, offs, perr, stable, s);
-            else part_pass<8>(kin, n, kind, shift, dbits, m, counts, offs, perr, stable, s);
+            // The second digit pass keeps the first one's order.
+            const bool second = ps > 0;
+            if (kw == 4) part_pass<4>(kin, n, kind, shift, dbits, m, counts, offs, perr, second, s);
+            else part_pass<8>(kin, n, kind, shift, dbits, m, counts, offs, perr, second, s);
             shift += dbits;
         }
     }
@@ -974,6 +960,7 @@ void partition_groupby(const col& key_in, const agg_plan& p, gx_groupby_hint* hi
     GX_LAUNCHED();
     exclusive_scan_i64(ucount.get<int64_t>(), uoff.get<int64_t>(), P, s);
     int64_t max_units = P + ceil_div(n, T) + 1;
+    const bool many_units = std::max<int64_t>(P, ceil_div(n, T)) >= 2 * (int64_t)dev().sm_count;
     dbuf units((size_t)max_units * sizeof(unit), s);
     k_unit_fill<<<(unsigned)ceil_div(P, 256), 256, 0, s>>>(pstart.get<int64_t>(), uoff.get<int64_t>(), P, T,
                                                            units.get<unit>());
@@ -1020,7 +1007,8 @@ void partition_groupby(const col& key_in, const agg_plan& p, gx_groupby_hint* hi
             for (int c = 0; c < d.n_cols; ++c) pd.col_ptr[c] = mc.out[c + 1];
             done_units = hash_units_aggregate(mc.out[0], kw, kind, pd, units.get<part_unit>(), uoff.get<int64_t>() + P,
                                               ceil_div(bound, (int64_t)P), R, grec.get<uint64_t>(), gcap,
-                                              flags.get<int>(), orec, ocount, rec_cap, rec_ovf, s);
+                                              flags.get<int>(), orec, ocount, rec_cap, rec_ovf, s, false,
+                                              many_units ? ceil_div(n, (int64_t)P) : 0);
         }
         if (n > 0 && !done_units) {
             size_t smem = (size_t)S * per_slot;

@@ -410,3 +410,24 @@ def test_partition_groups_per_partition_override(monkeypatch):
     got, exp, hint = run_both(key, [val], [(0, gx.SUM), (0, gx.COUNT_ALL)], gx.PARTITION, bound=1 << 16)
     assert hint.radix_bits == 12
     assert_columns_match(got, exp)
+
+
+@pytest.mark.parametrize("n", [70_001, 4096 * 37 + 5, 300_000])
+@pytest.mark.parametrize("kdt", [np.int32, np.int64])
+@pytest.mark.parametrize("skew", [False, True])
+def test_partition_two_passes_small_units(n, kdt, skew):
+    # Two digit passes over short runs of the first digit (tiles of the second
+    # pass span several of them), hundreds of partitions of few rows (small
+    # unit CTAs), and, with skew, a hot key whose partition is split.
+    rng = np.random.default_rng(n)
+    G = 68_000
+    key = rng.integers(0, G, n).astype(kdt) * kdt(31_337 if kdt == np.int32 else 2**40 + 7)
+    if skew:
+        key[rng.integers(0, n, n // 2)] = key[0]
+    iv = rng.integers(-2**40, 2**40, n)
+    fv = rng.random(n)
+    for vals, reqs, oreqs in (([iv], [(0, gx.SUM), (0, gx.COUNT_ALL)], [(0, O.SUM), (0, O.COUNT_ALL)]),
+                              ([iv, fv], [(0, gx.SUM), (0, gx.MIN), (1, gx.SUM), (1, gx.MAX)],
+                               [(0, O.SUM), (0, O.MIN), (1, O.SUM), (1, O.MAX)])):
+        t = gx.groupby([to_dev(key)], [to_dev(v) for v in vals], reqs, gx.make_hint(gx.PARTITION, radix_bits=10))
+        assert_columns_match(sort_by_key(t.numpy_columns()), list(O.groupby(key, vals, oreqs)))
