@@ -44,6 +44,12 @@ void hash_join(const join_inputs& in, const gx_join_hint& hint, bool rowids_only
 void partition_hash_join(const join_inputs& in, const gx_join_hint& hint, bool rowids_only, cudaStream_t s,
                          gx_table* out);
 
+// One-pass join of unique integer build keys through a hash table (gx_join.cu).
+// Returns false, with no output, when the build keys are not unique integers
+// or memory is short: the caller takes another plan.
+bool unique_hash_join(const join_inputs& in, const gx_join_hint& hint, bool rowids_only, bool build_left,
+                      cudaStream_t s, gx_table* out);
+
 #ifdef __CUDACC__
 __device__ __forceinline__ uint64_t ld_w(const void* p, int w, int64_t i) {
     switch (w) {

@@ -14,7 +14,8 @@
 // order.
 //
 // B200 design:
-//   * HASH: one open-addressing multiset of (key, build row) records at load
+//   * HASH: unique integer build keys go through unique_hash_join (gx_join.cu,
+//     one probe pass); otherwise one open-addressing multiset of (key, build row) records at load
 //     <= 1/2, built with one 64-bit compare-and-swap per row (4-byte keys
 //     pack key and row in one record; 8-byte keys claim the row word and then
 //     store the key), probed in 2048-row tiles: a count kernel sizes every
@@ -251,6 +252,8 @@ void hash_join(const join_inputs& in, const gx_join_hint& hint, bool rowids_only
     const int kw = size_of(in.lkey.type), kind = vkind_of(in.lkey.type);
     const int64_t nb = sd.bkey->n, np = sd.pkey->n;
     require(nb < (int64_t)0x7FFFFFFF, "hash join: the build side (smaller input) must have fewer than 2^31 rows");
+    // Unique integer build keys: one probe pass instead of count and write.
+    if (unique_hash_join(in, hint, rowids_only, sd.build_left, s, out)) return;
     const uint64_t cap = next_pow2((uint64_t)std::max<int64_t>(64, 2 * nb));
     const int64_t words = (int64_t)cap * (kw == 4 ? 1 : 2);
     dbuf table((size_t)words * 8, s);

@@ -117,3 +117,45 @@ def test_max_out_is_enforced(algo):
     x = np.arange(100, dtype=np.int32)
     with pytest.raises(gx.GxError):
         gx.inner_eq_join([to_dev(x), to_dev(x)], [to_dev(x), to_dev(x)], gx.make_join_hint(algo, gx.MAT_GFUR, max_out=50))
+
+
+@pytest.mark.parametrize("algo", [gx.JOIN_SORT, gx.JOIN_HASH])
+@pytest.mark.parametrize("kdt", [np.int32, np.uint32, np.int64, np.uint64])
+@pytest.mark.parametrize("nb,npr", [(1, 1), (3, 2049), (5000, 2048 * 3), (20_000, 70_001)])
+def test_unique_sparse_keys_one_pass(algo, kdt, nb, npr):
+    # Unique build keys too sparse for direct placement: slots with the row id
+    # or the single payload (4 or 8 bytes), few and many matches (buffers given
+    # back when under half is used), keys at the type's limits and equal to the
+    # empty slots' markers, and one duplicated key (another plan then).
+    rng = np.random.default_rng(nb)
+    lim = np.iinfo(kdt)
+    special = np.array([lim.max, lim.min, 0, lim.max - 1], kdt)
+    special = np.concatenate([special, np.array([-1], np.int64).astype(kdt),
+                              np.array([-2**63], np.int64).astype(kdt) if np.dtype(kdt).itemsize == 8 else special[:1]])
+    pool = np.unique(np.concatenate([special, rng.integers(lim.min, lim.max, 2 * nb, dtype=kdt)]))
+    for with_special in (False, True):
+        body = np.setdiff1d(pool, special)
+        bk = rng.permutation(body)[:nb]
+        if with_special and nb > 6:
+            bk[: len(np.unique(special))] = np.unique(special)
+        for dup in (False, True):
+            if dup and nb > 1:
+                bk = bk.copy()
+                bk[-1] = bk[0]
+            for share in (0.95, 0.05):
+                pk = np.where(rng.random(npr) < share, bk[rng.integers(0, nb, npr)],
+                              rng.integers(lim.min, lim.max, npr, dtype=kdt))
+                pk[: min(npr, 6)] = special[: min(npr, 6)]
+                el, er = O.join_pairs(bk, pk)
+                l, r = rowid_pairs(bk, pk, algo)
+                assert np.array_equal(l, el) and np.array_equal(r, er)
+                for pdt in (np.int64, np.float32, np.int16):
+                    bp, pp = np.arange(nb).astype(pdt), np.arange(npr).astype(np.int64)
+                    t = gx.inner_eq_join([to_dev(bk), to_dev(bp)], [to_dev(pk), to_dev(pp)],
+                                         gx.make_join_hint(algo, gx.MAT_GFUR))
+                    key, b, p = t.numpy_columns()
+                    o = np.lexsort((b, p))
+                    e = np.lexsort((bp[el], er))
+                    swap = nb > npr
+                    assert not swap and np.array_equal(p[o], er[e]) and np.array_equal(b[o], bp[el][e])
+                    assert np.array_equal(key[o], pk[er[e]])
