@@ -258,9 +258,14 @@ __device__ __forceinline__ int64_t find_or_insert(const batch_dev& b, const inst
 // Four 256-thread blocks per SM (at most 64 registers): the kernel waits on
 // dependent L2 accesses (offsets, string words, table entry, representative
 // row), so resident warps matter more than registers.
-__global__ void __launch_bounds__(256, 4) k_batch_main(batch_dev b) {
+constexpr int BM_NT = 256, BM_WARPS = BM_NT / 32;
+constexpr int BM_DATES = 4;  // dates a lane reads together
+__global__ void __launch_bounds__(BM_NT, 4) k_batch_main(batch_dev b) {
     __shared__ long long s_item;
     __shared__ inst_dev s_in;
+    __shared__ unsigned s_queue[BM_WARPS][31 + 32 * BM_DATES];  // kept rows of a warp, relative to the item
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    unsigned* queue = s_queue[warp];
     for (;;) {
         if (threadIdx.x == 0) {
             unsigned long long w = atomicAdd(b.work_counter, 1ull);
@@ -276,31 +281,19 @@ __global__ void __launch_bounds__(256, 4) k_batch_main(batch_dev b) {
         if (threadIdx.x == 0) s_in = b.inst[it.inst];
         __syncthreads();
         const inst_dev& in = s_in;
-        // A row's offsets, date and amount are loaded one iteration ahead,
-        // so the dependent chain of a row starts at its string bytes.
-        int64_t r = it.begin + threadIdx.x;
-        int64_t o0 = 0, o1 = 0, am = 0;
-        int32_t dt = 0;
-        if (r < it.end) {
-            o0 = in.offsets[r];
-            o1 = in.offsets[r + 1];
-            dt = in.date[r];
-            am = in.amount[r];
-        }
-        for (; r < it.end; r += blockDim.x) {
-            const int64_t rn = r + blockDim.x;
-            int64_t n0 = 0, n1 = 0, nam = 0;
-            int32_t ndt = 0;
-            if (rn < it.end) {
-                n0 = in.offsets[rn];
-                n1 = in.offsets[rn + 1];
-                ndt = in.date[rn];
-                nam = in.amount[rn];
-            }
-            // The date range is applied before the string is encoded: the
-            // output covers kept rows only, so a dropped row needs no hash,
-            // probe or string bytes (its codes would never be read).
-            if (dt >= in.lo && dt < in.hi) {
+        // The date range is applied before the string is encoded: the output
+        // covers kept rows only, so a dropped row needs no hash, probe or
+        // string bytes (its codes would never be read).  The kept rows of a
+        // warp are queued and taken 32 at a time, so every lane works through
+        // the dependent chain of a row (offsets, string words, table entry,
+        // key store, sums) instead of the kept share of them.
+        int fill = 0;
+        auto take = [&](int n) {  // the last n <= 32 queued rows
+            fill -= n;
+            if (lane < n) {
+                const int64_t r = it.begin + queue[fill + lane];
+                const int64_t o0 = in.offsets[r], o1 = in.offsets[r + 1];
+                const int64_t am = in.amount[r];
                 bool ins;
                 const int64_t slot = find_or_insert<true>(b, in, it.inst, r, o0, o1 - o0, &ins);
                 if (slot >= 0) {
@@ -308,11 +301,28 @@ __global__ void __launch_bounds__(256, 4) k_batch_main(batch_dev b) {
                     atomicAdd(&b.cnt_slot[slot], 1ull);
                 }
             }
-            o0 = n0;
-            o1 = n1;
-            dt = ndt;
-            am = nam;
+            __syncwarp();
+        };
+        const int rows = (int)(it.end - it.begin);
+        for (int r0 = warp * 32 * BM_DATES; r0 < rows; r0 += BM_WARPS * 32 * BM_DATES) {
+            int32_t dt[BM_DATES];
+#pragma unroll
+            for (int q = 0; q < BM_DATES; ++q) {
+                const int r = r0 + q * 32 + lane;
+                dt[q] = r < rows ? __ldg(in.date + it.begin + r) : 0;
+            }
+#pragma unroll
+            for (int q = 0; q < BM_DATES; ++q) {
+                const int r = r0 + q * 32 + lane;
+                const bool keep = r < rows && dt[q] >= in.lo && dt[q] < in.hi;
+                const unsigned m = __ballot_sync(0xffffffffu, keep);
+                if (keep) queue[fill + __popc(m & ((1u << lane) - 1u))] = (unsigned)r;
+                fill += __popc(m);
+            }
+            __syncwarp();
+            while (fill >= 32) take(32);
         }
+        take(fill);
     }
 }
 
@@ -596,7 +606,7 @@ static void batch_enqueue(gx_batch_plan* p, cudaStream_t s, bool count_launches 
     GX_CUDA(cudaMemsetAsync(p->out_first.get(), 0xFF, total_codes * 8, s));
     GX_CUDA(cudaMemsetAsync(p->out_groups.get(), 0, (size_t)n * 8, s));
     batch_dev b = batch_view(p);
-    k_batch_main<<<dev().sm_count * 8, 256, 0, s>>>(b);
+    k_batch_main<<<dev().sm_count * 8, BM_NT, 0, s>>>(b);
     GX_CUDA(cudaGetLastError());
     k_batch_finalize<<<grid_for((int64_t)std::max<size_t>(total_codes, 1), 256, 8), 256, 0, s>>>(b, n);
     GX_CUDA(cudaGetLastError());
