@@ -221,9 +221,8 @@ __global__ void __launch_bounds__(EMIT_NT) k_emit_write(emit_args a, const int64
 
 }  // namespace
 
-void emit_groupby_output(const agg_plan& p, const uint64_t* recs, int64_t nrec, bool compact,
-                         uint64_t empty_key, int64_t sentinel_rec, const int* sentinel_flag,
-                         int key_type, int64_t out_capacity, cudaStream_t s, gx_table* out) {
+static emit_args emit_records(const agg_plan& p, const uint64_t* recs, int64_t nrec, bool compact, uint64_t empty_key,
+                              int64_t sentinel_rec, const int* sentinel_flag) {
     emit_args a;
     std::memset(&a, 0, sizeof(a));
     a.recs = recs;
@@ -233,19 +232,17 @@ void emit_groupby_output(const agg_plan& p, const uint64_t* recs, int64_t nrec, 
     a.empty_key = empty_key;
     a.sentinel_rec = sentinel_rec;
     a.sentinel_flag = sentinel_flag;
-    a.key_width = size_of(key_type);
     a.count_word = p.d.count_word;
+    return a;
+}
+
+static int64_t emit_blocks(int64_t nrec) { return ceil_div(nrec > 0 ? nrec : 1, EMIT_NT); }
+
+// Output columns of `groups` rows, written from the records.
+static void emit_columns(const agg_plan& p, emit_args a, const int64_t* blk_off, int64_t groups, int64_t cap,
+                         int key_type, cudaStream_t s, gx_table* out) {
+    a.key_width = size_of(key_type);
     a.n_out = (int)p.outs.size();
-    int64_t nblk = ceil_div(nrec > 0 ? nrec : 1, EMIT_NT);
-    dbuf blk(nblk * sizeof(int64_t), s), off((nblk + 1) * sizeof(int64_t), s);
-    int64_t groups = nrec;
-    if (compact) {
-        k_emit_count<<<(unsigned)nblk, EMIT_NT, 0, s>>>(a, blk.get<int64_t>());
-        GX_LAUNCHED();
-        exclusive_scan_i64(blk.get<int64_t>(), off.get<int64_t>(), nblk, s);
-        groups = read_scalar(off.get<int64_t>() + nblk, s);
-    }
-    int64_t cap = std::max<int64_t>(groups, std::min<int64_t>(out_capacity, groups));
     out->cols.clear();
     out->cols.push_back(make_col(key_type, groups, s, cap));
     a.key_out = out->cols.back().buf.get();
@@ -259,9 +256,43 @@ void emit_groupby_output(const agg_plan& p, const uint64_t* recs, int64_t nrec, 
         a.out_lane_kind[o] = os.acc >= 0 ? p.d.acc_kind[os.acc] : VK_I;
     }
     if (groups > 0) {
-        k_emit_write<<<(unsigned)nblk, EMIT_NT, 0, s>>>(a, off.get<int64_t>());
+        k_emit_write<<<(unsigned)emit_blocks(a.nrec), EMIT_NT, 0, s>>>(a, blk_off);
         GX_LAUNCHED();
     }
+}
+
+int64_t emit_ctl_words(int64_t nrec) { return 2 * emit_blocks(nrec) + 1; }
+int64_t emit_total_word(int64_t nrec) { return 2 * emit_blocks(nrec); }
+
+void emit_place(const agg_plan& p, const uint64_t* recs, int64_t nrec, uint64_t empty_key, int64_t sentinel_rec,
+                const int* sentinel_flag, int64_t* ctl, cudaStream_t s) {
+    const int64_t nblk = emit_blocks(nrec);
+    const emit_args a = emit_records(p, recs, nrec, true, empty_key, sentinel_rec, sentinel_flag);
+    k_emit_count<<<(unsigned)nblk, EMIT_NT, 0, s>>>(a, ctl);
+    GX_LAUNCHED();
+    exclusive_scan_i64(ctl, ctl + nblk, nblk, s);
+}
+
+void emit_placed(const agg_plan& p, const uint64_t* recs, int64_t nrec, uint64_t empty_key, int64_t sentinel_rec,
+                 const int* sentinel_flag, const int64_t* ctl, int64_t groups, int key_type, cudaStream_t s,
+                 gx_table* out) {
+    emit_columns(p, emit_records(p, recs, nrec, true, empty_key, sentinel_rec, sentinel_flag),
+                 ctl + emit_blocks(nrec), groups, groups, key_type, s, out);
+}
+
+void emit_groupby_output(const agg_plan& p, const uint64_t* recs, int64_t nrec, bool compact,
+                         uint64_t empty_key, int64_t sentinel_rec, const int* sentinel_flag,
+                         int key_type, int64_t out_capacity, cudaStream_t s, gx_table* out) {
+    if (compact) {
+        dbuf ctl((size_t)emit_ctl_words(nrec) * 8, s);
+        emit_place(p, recs, nrec, empty_key, sentinel_rec, sentinel_flag, ctl.get<int64_t>(), s);
+        const int64_t groups = read_scalar(ctl.get<int64_t>() + emit_total_word(nrec), s);
+        emit_placed(p, recs, nrec, empty_key, sentinel_rec, sentinel_flag, ctl.get<int64_t>(), groups, key_type, s, out);
+        return;
+    }
+    const int64_t cap = std::max<int64_t>(nrec, std::min<int64_t>(out_capacity, nrec));
+    emit_columns(p, emit_records(p, recs, nrec, false, empty_key, sentinel_rec, sentinel_flag), nullptr, nrec, cap,
+                 key_type, s, out);
 }
 
 }  // namespace gx

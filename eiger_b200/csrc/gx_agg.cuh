@@ -83,6 +83,18 @@ void emit_groupby_output(const agg_plan& p, const uint64_t* recs, int64_t nrec, 
                          uint64_t empty_key, int64_t sentinel_rec, const int* sentinel_flag,
                          int key_type, int64_t out_capacity, cudaStream_t s, gx_table* out);
 
+// The compacting form in two halves, so that a caller reads the group count
+// together with its own flags: emit_place queues the count and scan of the
+// live records in `ctl` (emit_ctl_words words; word emit_total_word becomes
+// the group count), emit_placed allocates the columns and writes them.
+int64_t emit_ctl_words(int64_t nrec);
+int64_t emit_total_word(int64_t nrec);
+void emit_place(const agg_plan& p, const uint64_t* recs, int64_t nrec, uint64_t empty_key, int64_t sentinel_rec,
+                const int* sentinel_flag, int64_t* ctl, cudaStream_t s);
+void emit_placed(const agg_plan& p, const uint64_t* recs, int64_t nrec, uint64_t empty_key, int64_t sentinel_rec,
+                 const int* sentinel_flag, const int64_t* ctl, int64_t groups, int key_type, cudaStream_t s,
+                 gx_table* out);
+
 #ifdef __CUDACC__
 namespace dev_ {
 

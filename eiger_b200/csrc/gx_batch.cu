@@ -35,7 +35,6 @@ struct gx_batch_plan;
 
 namespace gx {
 
-void hash_groupby(const col& key, const agg_plan& p, gx_groupby_hint* hint, cudaStream_t s, gx_table* out);
 
 namespace {
 

@@ -346,12 +346,15 @@ inline int ilog2_ceil(uint64_t x) {
 inline uint64_t next_pow2(uint64_t x) { return x <= 1 ? 1 : (uint64_t(1) << ilog2_ceil(x)); }
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-// Host <- device copy of a small value with a stream sync.
+// Host <- device copy of at most HOST_READ_MAX bytes through the calling
+// thread's pinned buffer, with a stream sync (a pageable destination makes the
+// driver bounce the copy through its own).
+constexpr size_t HOST_READ_MAX = 4096;
+void host_read(void* dst, const void* dptr, size_t bytes, cudaStream_t s);
 template <typename T>
 T read_scalar(const T* dptr, cudaStream_t s) {
     T v;
-    GX_CUDA(cudaMemcpyAsync(&v, dptr, sizeof(T), cudaMemcpyDeviceToHost, s));
-    GX_CUDA(cudaStreamSynchronize(s));
+    host_read(&v, dptr, sizeof(T), s);
     return v;
 }
 

@@ -358,8 +358,7 @@ void dictionary_encode(const gx_column_view& v, int encode_type, int64_t size_hi
             GX_LAUNCHED();
         }
         int hflags[4];
-        GX_CUDA(cudaMemcpyAsync(hflags, tb.flags.get(), 16, cudaMemcpyDeviceToHost, s));
-        GX_CUDA(cudaStreamSynchronize(s));
+        host_read(hflags, tb.flags.get(), 16, s);
         if (hflags[0]) continue;
         unsigned long long ndv_u;
         std::memcpy(&ndv_u, &hflags[2], 8);

@@ -17,29 +17,36 @@ namespace gx {
 // and writes the suggested radix bits.
 int selector_choose(const col& key, const agg_plan& plan, int* radix_bits, cudaStream_t s);
 
-static void auto_select(const gx_table_view* key, const gx_table_view* val, const gx_agg_request* req, int nreq,
-                        gx_groupby_hint* hint, cudaStream_t s) {
-    if (hint->groupby_algo != GX_GB_AUTO) return;
+// Returns the key column's distinct estimate when the rule took one, else -1.
+static int64_t auto_select(const gx_table_view* key, const gx_table_view* val, const gx_agg_request* req, int nreq,
+                           gx_groupby_hint* hint, cudaStream_t s) {
+    if (hint->groupby_algo != GX_GB_AUTO) return -1;
     for (int64_t i = 0; i < key->num_columns; ++i)
-        if (key->columns[i].type == GX_STRING) { hint->groupby_algo = GX_GB_HASH; return; }
-    if (key->num_columns != 1) { hint->groupby_algo = GX_GB_HASH; return; }
+        if (key->columns[i].type == GX_STRING) { hint->groupby_algo = GX_GB_HASH; return -1; }
+    if (key->num_columns != 1) { hint->groupby_algo = GX_GB_HASH; return -1; }
     col k = resolve(key->columns[0]);
     if (hint->selector == GX_SELECT_LEARNED) {
         int bits = 0;
         const agg_plan plan = make_agg_plan(val, req, nreq, hint->agg_count != 0);
         hint->groupby_algo = selector_choose(k, plan, &bits, s);
         if (hint->radix_bits <= 0) hint->radix_bits = bits;
-        return;
+        return -1;
     }
-    int64_t est = ndv_estimate(k, s);
-    bool four = size_of(k.type) == 4;
-    int64_t thr = four ? (int64_t(1) << 14) : (int64_t(1) << 18);
+    const bool four = size_of(k.type) == 4;
+    const int64_t thr = four ? (int64_t(1) << 14) : (int64_t(1) << 18);
+    if (k.n <= thr / 2) {  // no estimate of so few rows comes near the threshold
+        hint->groupby_algo = GX_GB_HASH;
+        return -1;
+    }
+    const int64_t est = ndv_estimate(k, s);
     hint->groupby_algo = est <= thr ? GX_GB_HASH : GX_GB_PARTITION;
+    return est;
 }
 
-// One numeric key column through the chosen variant.
+// One numeric key column through the chosen variant (ndv: its distinct estimate
+// when already taken).
 static void groupby_single(const col& k, const gx_table_view* val, const gx_agg_request* req, int nreq,
-                           gx_groupby_hint* hint, cudaStream_t s, gx_table* out) {
+                           gx_groupby_hint* hint, cudaStream_t s, gx_table* out, int64_t ndv = -1) {
     require(is_numeric(k.type), "groupby: unsupported key type " + type_name(k.type));
     agg_plan p = make_agg_plan(val, req, nreq, hint->agg_count != 0);
     switch (hint->groupby_algo) {
@@ -49,9 +56,9 @@ static void groupby_single(const col& k, const gx_table_view* val, const gx_agg_
             break;
         case GX_GB_SORT: sort_groupby(k, p, hint, false, s, out); break;
         case GX_GB_SORT_GFUR: sort_groupby(k, p, hint, true, s, out); break;
-        case GX_GB_PARTITION: partition_groupby(k, p, hint, false, s, out); break;
-        case GX_GB_PARTITION_GFUR: partition_groupby(k, p, hint, true, s, out); break;
-        case GX_GB_HASH: hash_groupby(k, p, hint, s, out); break;
+        case GX_GB_PARTITION: partition_groupby(k, p, hint, false, s, out, ndv); break;
+        case GX_GB_PARTITION_GFUR: partition_groupby(k, p, hint, true, s, out, ndv); break;
+        case GX_GB_HASH: hash_groupby(k, p, hint, s, out, ndv); break;
         default: fail(GX_EINVAL, "Unsupported groupby algorithm");
     }
 }
@@ -108,13 +115,13 @@ void groupby_dispatch(const gx_table_view* key, const gx_table_view* val, const 
                                                    " has a different row count than the key");
 
     if (forced_algo >= 0) hint->groupby_algo = forced_algo;
-    auto_select(key, val, req, nreq, hint, s);
+    const int64_t ndv = auto_select(key, val, req, nreq, hint, s);
     bool str = false;
     for (int64_t i = 0; i < key->num_columns; ++i) str |= key->columns[i].type == GX_STRING;
     const bool composite = str || key->num_columns > 1;
     if (hint->allow_hash_fallback && hint->groupby_algo != GX_GB_HASH && composite) hint->groupby_algo = GX_GB_HASH;
     if (!composite) {
-        groupby_single(resolve(key->columns[0]), val, req, nreq, hint, s, out);
+        groupby_single(resolve(key->columns[0]), val, req, nreq, hint, s, out, ndv);
         GX_CUDA(cudaStreamSynchronize(s));
         return;
     }

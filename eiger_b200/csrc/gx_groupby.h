@@ -6,7 +6,9 @@
 namespace gx {
 
 // ----- hash group-by (gx_groupby_hash.cu) -----
-void init_records(uint64_t* recs, int64_t nrec, const agg_desc& d, uint64_t empty, cudaStream_t s);
+// Also zeroes the flag words (when given).
+void init_records(uint64_t* recs, int64_t nrec, const agg_desc& d, uint64_t empty, cudaStream_t s,
+                  uint64_t* flags = nullptr, int nflags = 0);
 int hash_smem_slots(const agg_desc& d, int key_width, int64_t groups_bound, int* replicas);
 // Sample sketch of a key column (gx_selector.cu): f[6..13] are the shares of
 // the 8 most frequent keys in a 2^14-row strided sample.
@@ -17,6 +19,13 @@ struct part_unit {
     int64_t begin, end;
     int split, pad;
 };
+// The units of hash_units_aggregate: a device list of *n_list units, or, with
+// list null, equal ranges of `rows` rows, `step` each, every one split.
+struct unit_source {
+    const part_unit* list;
+    const int64_t* n_list;
+    int64_t rows, step;
+};
 // Aggregates partitioned rows unit by unit in shared-memory tables (the hash
 // group-by's table code); `shift` = partition bits of the key hash, gpp =
 // expected groups per partition.  Final groups of whole, unspilled units are
@@ -26,18 +35,18 @@ struct part_unit {
 // dense_only: only the dense-id kernel (false when the plan has no compiled
 // form or its tables do not fit).  unit_rows: mean rows per partition (0: not
 // known), which decides the size of the dense-id kernel's CTAs.
-bool hash_units_aggregate(const void* keys, int kw, int kind, const agg_desc& d, const part_unit* units,
-                          const int64_t* n_units, int64_t gpp, int shift, uint64_t* grec, uint64_t gcap, int* gflags,
+bool hash_units_aggregate(const void* keys, int kw, int kind, const agg_desc& d, const unit_source& units, int64_t gpp, int shift, uint64_t* grec, uint64_t gcap, int* gflags,
                           uint64_t* orec, unsigned long long* ocount, int64_t rec_cap, int* rec_ovf, cudaStream_t s,
                           bool dense_only = false, int64_t unit_rows = 0);
+// ndv: distinct estimate of the key column when already taken, else -1.
 void hash_groupby(const col& key, const agg_plan& p, gx_groupby_hint* hint, cudaStream_t s,
-                  gx_table* out);
+                  gx_table* out, int64_t ndv = -1);
 
 // ----- sort / partition group-by (gx_groupby_sort.cu, gx_groupby_partition.cu) -----
 void sort_groupby(const col& key, const agg_plan& p, gx_groupby_hint* hint, bool gfur,
                   cudaStream_t s, gx_table* out);
 void partition_groupby(const col& key, const agg_plan& p, gx_groupby_hint* hint, bool gfur,
-                       cudaStream_t s, gx_table* out);
+                       cudaStream_t s, gx_table* out, int64_t ndv = -1);
 
 // Radix-partitions (key, row id) by R bits of the partition hash; see
 // gx_groupby_partition.cu.

@@ -314,10 +314,22 @@ __global__ void __launch_bounds__(HGB_NT, 1) k_hash_groupby(const void* __restri
 // never overflowed its table appends its final groups densely; a split (or
 // spilled) unit merges into the global table like k_hash_groupby's CTAs.
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ int64_t unit_count(const unit_source& us) {
+    return us.list ? *us.n_list : (us.rows + us.step - 1) / us.step;
+}
+__device__ __forceinline__ part_unit unit_at(const unit_source& us, int64_t u) {
+    if (us.list) return us.list[u];
+    part_unit x;
+    x.begin = u * us.step;
+    x.end = min(us.rows, x.begin + us.step);
+    x.split = 1;
+    x.pad = 0;
+    return x;
+}
+
 template <int KW, int NV, class... ACCS>
 __global__ void __launch_bounds__(HGB_NT, 1) k_hash_units(const void* __restrict__ keys, int key_kind, agg_desc d,
-                                                           const part_unit* __restrict__ units,
-                                                           const int64_t* __restrict__ n_units, uint32_t s_slots,
+                                                           unit_source us, uint32_t s_slots,
                                                            int reps, int shift, gtable g,
                                                            uint64_t* __restrict__ out_recs,
                                                            unsigned long long* __restrict__ out_count,
@@ -347,9 +359,9 @@ __global__ void __launch_bounds__(HGB_NT, 1) k_hash_units(const void* __restrict
     const int rep = (int)(threadIdx.x % (unsigned)reps);
     unsigned* my_counts = st.counts + rep;
     uint64_t* my_acc = st.acc + rep;
-    const int64_t nu = *n_units;
+    const int64_t nu = unit_count(us);
     for (int64_t u = blockIdx.x; u < nu; u += gridDim.x) {
-        const part_unit un = units[u];
+        const part_unit un = unit_at(us, u);
         for (uint32_t i = threadIdx.x; i < s_slots; i += HGB_NT) st.keys[i] = EMPTY;
         for (uint32_t i = threadIdx.x; i < s_slots * reps; i += HGB_NT) st.counts[i] = 0;
         for (int a = 0; a < d.n_acc; ++a) {
@@ -656,8 +668,7 @@ __device__ __forceinline__ uint64_t ud_load_key(const void* keys, int64_t i, int
 
 template <int NT, int KW, int NV, class... ACCS>
 __global__ void __launch_bounds__(NT, NT == HGB_NT ? 1 : 4) k_units_dense(const void* __restrict__ keys, int key_kind, agg_desc d,
-                                                            const part_unit* __restrict__ units,
-                                                            const int64_t* __restrict__ n_units, uint32_t s_slots,
+                                                            unit_source us, uint32_t s_slots,
                                                             uint32_t gcap, int reps, uint32_t gpp, int shift,
                                                             gtable g, uint64_t* __restrict__ out_recs,
                                                             unsigned long long* __restrict__ out_count,
@@ -696,9 +707,9 @@ __global__ void __launch_bounds__(NT, NT == HGB_NT ? 1 : 4) k_units_dense(const 
         if constexpr (CP) spec::apply_all<0, ACCS...>(ma, (uint32_t)GR, at, vv);
         else dev_::shared_row_update<NV>(ma, GR, (int)at, d, vv);
     };
-    const int64_t nu = *n_units;
+    const int64_t nu = unit_count(us);
     for (int64_t u = blockIdx.x; u < nu; u += gridDim.x) {
-        const part_unit un = units[u];
+        const part_unit un = unit_at(us, u);
         // Replicas of this unit: every one for a piece of a split (large)
         // partition, where a few groups take most rows; otherwise one per 16
         // rows of a group, since each replica also costs set-up and merge
@@ -850,7 +861,8 @@ __global__ void __launch_bounds__(NT, NT == HGB_NT ? 1 : 4) k_units_dense(const 
 
 // Initialise `nrec` records: key word = empty, count 0, accumulators = identity.
 __global__ void k_init_records(uint64_t* __restrict__ recs, int64_t nrec, int rec_words, uint64_t empty,
-                               agg_desc d) {
+                               agg_desc d, uint64_t* __restrict__ flags, int nflags) {
+    if (blockIdx.x == 0 && (int)threadIdx.x < nflags) flags[threadIdx.x] = 0;
     int64_t total = nrec * rec_words;
     for (int64_t w = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; w < total;
          w += (int64_t)gridDim.x * blockDim.x) {
@@ -869,9 +881,11 @@ __global__ void k_init_records(uint64_t* __restrict__ recs, int64_t nrec, int re
 
 }  // namespace
 
-void init_records(uint64_t* recs, int64_t nrec, const agg_desc& d, uint64_t empty, cudaStream_t s) {
+void init_records(uint64_t* recs, int64_t nrec, const agg_desc& d, uint64_t empty, cudaStream_t s, uint64_t* flags,
+                  int nflags) {
     if (nrec <= 0) return;
-    k_init_records<<<grid_for(nrec * d.rec_words, 256, 8), 256, 0, s>>>(recs, nrec, d.rec_words, empty, d);
+    k_init_records<<<grid_for(nrec * d.rec_words, 256, 8), 256, 0, s>>>(recs, nrec, d.rec_words, empty, d, flags,
+                                                                         nflags);
     GX_LAUNCHED();
 }
 
@@ -962,8 +976,7 @@ static void launch_hash(bool smem_mode, int nv, int grid, size_t smem, cudaStrea
 struct units_args {
     const void* keys;
     int kind;
-    const part_unit* units;
-    const int64_t* n_units;
+    unit_source units;
     uint32_t slots;
     int reps, shift;
     gtable g;
@@ -978,7 +991,7 @@ template <int KW, int NV, class... ACCS>
 static void launch_units(int grid, size_t smem, cudaStream_t s, const agg_desc& d, const units_args& a) {
     GX_CUDA(cudaFuncSetAttribute(k_hash_units<KW, NV, ACCS...>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem));
-    k_hash_units<KW, NV, ACCS...><<<grid, HGB_NT, smem, s>>>(a.keys, a.kind, d, a.units, a.n_units, a.slots, a.reps,
+    k_hash_units<KW, NV, ACCS...><<<grid, HGB_NT, smem, s>>>(a.keys, a.kind, d, a.units, a.slots, a.reps,
                                                              a.shift, a.g, a.orec, a.ocount, a.rec_cap, a.rec_ovf);
 }
 
@@ -994,7 +1007,7 @@ static void launch_units_dense_nt(int grid, size_t smem, cudaStream_t s, const a
                                   uint32_t gcap, uint32_t gpp) {
     GX_CUDA(cudaFuncSetAttribute(k_units_dense<NT, KW, NV, ACCS...>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem));
-    k_units_dense<NT, KW, NV, ACCS...><<<grid, NT, smem, s>>>(a.keys, a.kind, d, a.units, a.n_units, a.slots, gcap,
+    k_units_dense<NT, KW, NV, ACCS...><<<grid, NT, smem, s>>>(a.keys, a.kind, d, a.units, a.slots, gcap,
                                                               a.reps, gpp, a.shift, a.g, a.orec, a.ocount,
                                                               a.rec_cap, a.rec_ovf);
 }
@@ -1062,42 +1075,29 @@ static void units_dispatch(int grid, size_t smem, cudaStream_t s, const agg_desc
 // replicated accumulators, no atomics on the global table per row) and
 // merged into the global table once per range.
 static bool hash_groupby_units(const col& key, const agg_desc& d, int64_t groups, const gtable& g, cudaStream_t s) {
-    const int64_t n = key.n;
-    const int ns = dev().sm_count;
-    std::vector<part_unit> hu;
-    const int64_t per = ceil_div(n, (int64_t)ns);
-    for (int64_t b = 0; b < n; b += per) hu.push_back({b, std::min(n, b + per), 1, 0});
-    const int64_t nu = (int64_t)hu.size();
-    dbuf ub((size_t)nu * sizeof(part_unit) + 64, s);
-    int64_t* d_nu = reinterpret_cast<int64_t*>(ub.get<char>() + (size_t)nu * sizeof(part_unit));
-    GX_CUDA(cudaMemcpyAsync(ub.get(), hu.data(), (size_t)nu * sizeof(part_unit), cudaMemcpyHostToDevice, s));
-    GX_CUDA(cudaMemcpyAsync(d_nu, &nu, 8, cudaMemcpyHostToDevice, s));
-    // No unit is a whole partition, so no final records are appended.
-    uint64_t* no_rec = reinterpret_cast<uint64_t*>(d_nu + 1);
-    unsigned long long* no_cnt = reinterpret_cast<unsigned long long*>(d_nu + 2);
-    int* no_ovf = reinterpret_cast<int*>(d_nu + 3);
-    const bool ok = hash_units_aggregate(key.data, size_of(key.type), vkind_of(key.type), d, ub.get<part_unit>(), d_nu,
-                                         groups, 0, g.recs, g.mask + 1, g.sentinel_flag, no_rec, no_cnt, 0, no_ovf, s,
-                                         true);
-    if (ok) GX_CUDA(cudaStreamSynchronize(s));  // the unit list lives in this scope
-    return ok;
+    // Every unit is a piece of the whole, so no final records are appended.
+    const unit_source us{nullptr, nullptr, key.n, ceil_div(key.n, (int64_t)dev().sm_count)};
+    return hash_units_aggregate(key.data, size_of(key.type), vkind_of(key.type), d, us, groups, 0, g.recs, g.mask + 1,
+                                g.sentinel_flag, nullptr, nullptr, 0, nullptr, s, true);
 }
 
 static bool hash_groupby_run(const col& key, int out_key_type, const agg_plan& p, uint64_t cap, int smem_mode,
-                             int64_t units_groups, uint32_t s_slots, int reps, int64_t out_capacity, cudaStream_t s,
-                             gx_table* out) {
+                             int64_t units_groups, uint32_t s_slots, int reps, cudaStream_t s, gx_table* out) {
     const agg_desc& d = p.d;
     int kw = size_of(key.type);
     uint64_t empty = kw == 4 ? G_EMPTY4 : G_EMPTY8;
-    dbuf recs((cap + 1) * d.rec_words * sizeof(uint64_t), s);
-    dbuf flags(2 * sizeof(int), s);
-    GX_CUDA(cudaMemsetAsync(flags.get(), 0, 2 * sizeof(int), s));
-    init_records(recs.get<uint64_t>(), (int64_t)cap + 1, d, empty, s);
+    // Records, then the emission's counts and offsets, whose last word (the
+    // group count) and the flag word behind it are read together.
+    const int64_t nrec = (int64_t)cap + 1, rec_words = nrec * d.rec_words, ctl_words = emit_ctl_words(nrec);
+    dbuf recs((size_t)(rec_words + ctl_words + 1) * sizeof(uint64_t), s);
+    int64_t* ctl = recs.get<int64_t>() + rec_words;
+    int* flags = reinterpret_cast<int*>(ctl + ctl_words);
+    init_records(recs.get<uint64_t>(), nrec, d, empty, s, reinterpret_cast<uint64_t*>(flags), 1);
     gtable g;
     g.recs = recs.get<uint64_t>();
     g.mask = cap - 1;
-    g.sentinel_flag = flags.get<int>();
-    g.overflow = flags.get<int>() + 1;
+    g.sentinel_flag = flags;
+    g.overflow = flags + 1;
     int kind = vkind_of(key.type);
     const bool units = key.n > 0 && units_groups > 0 && hash_groupby_units(key, d, units_groups, g, s);
     if (key.n > 0 && !units) {
@@ -1112,17 +1112,18 @@ static bool hash_groupby_run(const col& key, int out_key_type, const agg_plan& p
         else launch_hash<8>(smem_mode, nv, grid, smem, s, key.data, key.n, kind, d, g, s_slots, reps);
         GX_LAUNCHED();
     }
+    emit_place(p, recs.get<uint64_t>(), nrec, empty, (int64_t)cap, flags, ctl, s);
+    int64_t h[2];  // group count; sentinel and overflow flags
+    host_read(h, ctl + emit_total_word(nrec), sizeof(h), s);
     int hflags[2];
-    GX_CUDA(cudaMemcpyAsync(hflags, flags.get(), sizeof(hflags), cudaMemcpyDeviceToHost, s));
-    GX_CUDA(cudaStreamSynchronize(s));
+    std::memcpy(hflags, &h[1], sizeof(hflags));
     if (hflags[1]) return false;
-    emit_groupby_output(p, recs.get<uint64_t>(), (int64_t)cap + 1, true, empty, (int64_t)cap,
-                        flags.get<int>(), out_key_type, out_capacity, s, out);
+    emit_placed(p, recs.get<uint64_t>(), nrec, empty, (int64_t)cap, flags, ctl, h[0], out_key_type, s, out);
     return true;
 }
 
 void hash_groupby(const col& key_in, const agg_plan& p, gx_groupby_hint* hint, cudaStream_t s,
-                  gx_table* out) {
+                  gx_table* out, int64_t ndv) {
     owned_col widened;
     col key = key_in;
     if (size_of(key.type) < 4) {
@@ -1135,7 +1136,7 @@ void hash_groupby(const col& key_in, const agg_plan& p, gx_groupby_hint* hint, c
     bool bound_known = hint->groups_upper_bound > 0 && hint->groups_upper_bound < n;
     if (!bound_known && n > (1 << 16)) {
         // No usable bound: size from a HyperLogLog estimate (+15% margin).
-        int64_t est = ndv_estimate(key, s);
+        int64_t est = ndv >= 0 ? ndv : ndv_estimate(key, s);
         bound = std::min<int64_t>(n, std::max<int64_t>(1024, est + est / 8 + 64));
     }
     int lf = hint->load_factor_pct > 0 ? hint->load_factor_pct : 50;
@@ -1167,17 +1168,14 @@ void hash_groupby(const col& key_in, const agg_plan& p, gx_groupby_hint* hint, c
                                          smem_mode && !getenv("GX_HASH_NO_UNITS")
                                      ? bound
                                      : 0;
-    int64_t out_cap = std::min<int64_t>(n, hint->groups_upper_bound > 0 ? hint->groups_upper_bound : n);
     for (int attempt = 0; attempt < 6; ++attempt) {
-        if (hash_groupby_run(key, key_in.type, p, cap, smem_mode, units_groups, s_slots, reps, out_cap, s, out))
-            return;
+        if (hash_groupby_run(key, key_in.type, p, cap, smem_mode, units_groups, s_slots, reps, s, out)) return;
         cap *= 4;
     }
     fail(GX_EOVERFLOW, "hash group-by table overflow after retries");
 }
 
-bool hash_units_aggregate(const void* keys, int kw, int kind, const agg_desc& d, const part_unit* units,
-                          const int64_t* n_units, int64_t gpp, int shift, uint64_t* grec, uint64_t gcap, int* gflags,
+bool hash_units_aggregate(const void* keys, int kw, int kind, const agg_desc& d, const unit_source& units, int64_t gpp, int shift, uint64_t* grec, uint64_t gcap, int* gflags,
                           uint64_t* orec, unsigned long long* ocount, int64_t rec_cap, int* rec_ovf, cudaStream_t s,
                           bool dense_only, int64_t unit_rows) {
     const size_t budget = 200 * 1024;
@@ -1215,7 +1213,7 @@ bool hash_units_aggregate(const void* keys, int kw, int kind, const agg_desc& d,
         size_t r = 16;
         while (r > 1 && need(r) > room) r >>= 1;
         if (need(r) <= room) {
-            const units_args a{keys, kind, units, n_units, dslots, (int)r, shift,
+            const units_args a{keys, kind, units, dslots, (int)r, shift,
                                gtable{grec, gcap - 1, gflags, gflags + 1}, orec, ocount, rec_cap, rec_ovf, small};
             const uint32_t g32 = (uint32_t)std::min<int64_t>(std::max<int64_t>(gpp, 1), ids);
             const int dgrid = small ? grid * 4 : grid;
@@ -1237,7 +1235,7 @@ bool hash_units_aggregate(const void* keys, int kw, int kind, const agg_desc& d,
     while (reps & (reps - 1)) reps &= reps - 1;
     const size_t smem = (((size_t)slots * kw + 15) & ~size_t(15)) + (((size_t)slots * 4 * reps + 15) & ~size_t(15)) +
                         (size_t)slots * reps * 8 * d.n_acc;
-    units_args a{keys, kind, units, n_units, slots, (int)reps, shift,
+    units_args a{keys, kind, units, slots, (int)reps, shift,
                  gtable{grec, gcap - 1, gflags, gflags + 1}, orec, ocount, rec_cap, rec_ovf, false};
     GX_PROF("partition_aggregate", s);
     if (kw == 4) units_dispatch<4>(grid, smem, s, d, a);

@@ -585,11 +585,12 @@ __global__ void k_starts_from_offsets(const int64_t* __restrict__ offs, int64_t 
 
 // Work units: partition p split into ceil(size/T) units.
 __global__ void k_unit_counts(const int64_t* __restrict__ part_start, int P, int64_t T,
-                              int64_t* __restrict__ ucount) {
+                              int64_t* __restrict__ ucount, int* __restrict__ n_split) {
     int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p < P) {
         int64_t sz = part_start[p + 1] - part_start[p];
         ucount[p] = sz == 0 ? 0 : (sz + T - 1) / T;
+        if (sz > T) atomicAdd(n_split, 1);
     }
 }
 using unit = part_unit;
@@ -847,7 +848,7 @@ void part_pass(const void* kin, int64_t n, int kind, int shift, int dbits, move_
 }  // namespace
 
 void partition_groupby(const col& key_in, const agg_plan& p, gx_groupby_hint* hint, bool gfur, cudaStream_t s,
-                       gx_table* out) {
+                       gx_table* out, int64_t ndv) {
     owned_col widened;
     col key = key_in;
     if (size_of(key.type) < 4) {
@@ -869,7 +870,7 @@ void partition_groupby(const col& key_in, const agg_plan& p, gx_groupby_hint* hi
     while (S_max > 256 && S_max * per_slot > 200 * 1024) S_max >>= 1;
     int64_t bound = std::min<int64_t>(n, hint->groups_upper_bound > 0 ? hint->groups_upper_bound : n);
     if (!(hint->groups_upper_bound > 0 && hint->groups_upper_bound < n) && n > (1 << 16))
-        bound = std::min<int64_t>(n, ndv_estimate(key, s) * 9 / 8 + 64);
+        bound = std::min<int64_t>(n, (ndv >= 0 ? ndv : ndv_estimate(key, s)) * 9 / 8 + 64);
     // About 256 groups per partition: a shared table of ~1K slots holds them
     // (with a few accumulator replicas), and up to 2^16 groups need a single
     // 8-bit radix pass.
@@ -909,8 +910,9 @@ void partition_groupby(const col& key_in, const agg_plan& p, gx_groupby_hint* hi
     int64_t ntiles = ceil_div(std::max<int64_t>(n, 1), PS_TILE);
     int64_t* counts = static_cast<int64_t*>(thread_scratch(SCRATCH_SLOTS - 2, (size_t)PS_BINS * ntiles * 8));
     int64_t* offs = static_cast<int64_t*>(thread_scratch(SCRATCH_SLOTS - 1, (size_t)PS_BINS * ntiles * 8 + 8));
-    // Unit offsets [0, P] then one word the bulk-copy scatter sets when a
-    // copy wait gave up, so one read after the unit setup fetches both.
+    // Unit offsets [0, P] then one word with the flag the bulk-copy scatter
+    // sets when a copy wait gave up and the number of split partitions, so one
+    // read after the unit setup fetches them.
     dbuf uoff((size_t)(P + 2) * 8, s);
     int* perr = reinterpret_cast<int*>(uoff.get<int64_t>() + P + 1);
     GX_CUDA(cudaMemsetAsync(perr, 0, 8, s));
@@ -956,7 +958,8 @@ void partition_groupby(const col& key_in, const agg_plan& p, gx_groupby_hint* hi
     // that about four units per SM exist.
     int64_t T = std::max<int64_t>(1 << 14, std::min<int64_t>(2 * ceil_div(n, P), ceil_div(n, (int64_t)dev().sm_count * 8)));
     dbuf ucount((size_t)P * 8, s);
-    k_unit_counts<<<(unsigned)ceil_div(P, 256), 256, 0, s>>>(pstart.get<int64_t>(), P, T, ucount.get<int64_t>());
+    k_unit_counts<<<(unsigned)ceil_div(P, 256), 256, 0, s>>>(pstart.get<int64_t>(), P, T, ucount.get<int64_t>(),
+                                                             perr + 1);
     GX_LAUNCHED();
     exclusive_scan_i64(ucount.get<int64_t>(), uoff.get<int64_t>(), P, s);
     int64_t max_units = P + ceil_div(n, T) + 1;
@@ -967,25 +970,27 @@ void partition_groupby(const col& key_in, const agg_plan& p, gx_groupby_hint* hi
     GX_LAUNCHED();
 
     uint64_t empty = kw == 4 ? PG_EMPTY4 : PG_EMPTY8;
-    // Split units merge through the spill table, so size it for every group
-    // when any partition was split; otherwise it only catches overflow.  When
-    // a table for every group is small (<= 64 MB) it is used either way, so
-    // the host does not wait for the unit count before the aggregation; the
-    // scatter's timeout flag is then read with the final flags.
+    // Split units merge through the spill table.  When a table for every group
+    // is small (<= 16 MB) it is used, so the host does not wait for the split
+    // count before the aggregation; the scatter's timeout flag is then read
+    // with the final flags.  Otherwise the table holds four times the groups
+    // that the split partitions are expected to have (their hash spreads
+    // groups evenly), or every group when partitions hold more than a shared
+    // table (radix bits forced low by the hint).  5*10^7 Zipf rows in 3*10^6
+    // groups: clearing and scanning 268 MB for every group took 0.15 ms, and
+    // allocating it stalled the stream pool for up to 40 ms.
     int64_t tail[2] = {0, 0};
-    const int64_t live_parts = std::min<int64_t>(P, n);
     const uint64_t all_groups = std::max<uint64_t>(1u << 16, next_pow2((uint64_t)bound * 2));
     uint64_t gcap = 1u << 16;
-    const bool tail_later = (all_groups + 1) * (uint64_t)d.rec_words * 8 <= (64ull << 20);
+    const bool tail_later = (all_groups + 1) * (uint64_t)d.rec_words * 8 <= (16ull << 20);
     if (tail_later) {
         gcap = all_groups;
     } else {
-        GX_CUDA(cudaMemcpyAsync(tail, uoff.get<int64_t>() + P, sizeof(tail), cudaMemcpyDeviceToHost, s));
-        GX_CUDA(cudaStreamSynchronize(s));
+        host_read(tail, uoff.get<int64_t>() + P, sizeof(tail), s);
         if ((int)tail[1]) fail(GX_ETIMEOUT, "partition scatter: a bulk copy into shared memory did not complete");
-        // Also when partitions hold more groups than a shared table (radix
-        // bits forced low by the hint): their overflow spills here.
-        if (tail[0] > live_parts || ceil_div(bound, (int64_t)P) > 512) gcap = all_groups;
+        const int64_t gpp_est = ceil_div(bound, (int64_t)P), n_split = tail[1] >> 32;
+        gcap = gpp_est > 512 ? all_groups
+                             : std::min(all_groups, std::max(gcap, next_pow2((uint64_t)(n_split * gpp_est * 4))));
     }
     int64_t out_cap = std::min<int64_t>(n, hint->groups_upper_bound > 0 ? hint->groups_upper_bound : n);
     // Output records: sized from the group bound, grown (up to n) on overflow.
@@ -993,8 +998,7 @@ void partition_groupby(const col& key_in, const agg_plan& p, gx_groupby_hint* hi
     for (int attempt = 0; attempt < 8; ++attempt) {
         dbuf grec((gcap + 1) * d.rec_words * 8, s);
         dbuf flags(32, s);  // [0] sentinel, [1] spill overflow, [8..15] count, [16] record overflow
-        GX_CUDA(cudaMemsetAsync(flags.get(), 0, 32, s));
-        init_records(grec.get<uint64_t>(), (int64_t)gcap + 1, d, empty, s);
+        init_records(grec.get<uint64_t>(), (int64_t)gcap + 1, d, empty, s, flags.get<uint64_t>(), 4);
         uint64_t* orec = static_cast<uint64_t*>(thread_scratch(SCRATCH_SLOTS - 3, (size_t)rec_cap * d.rec_words * 8));
         unsigned long long* ocount = reinterpret_cast<unsigned long long*>(flags.get<char>() + 8);
         int* rec_ovf = reinterpret_cast<int*>(flags.get<char>() + 16);
@@ -1005,7 +1009,8 @@ void partition_groupby(const col& key_in, const agg_plan& p, gx_groupby_hint* hi
             // hash-table kernel over the partitioned copies.
             agg_desc pd = d;
             for (int c = 0; c < d.n_cols; ++c) pd.col_ptr[c] = mc.out[c + 1];
-            done_units = hash_units_aggregate(mc.out[0], kw, kind, pd, units.get<part_unit>(), uoff.get<int64_t>() + P,
+            done_units = hash_units_aggregate(mc.out[0], kw, kind, pd,
+                                              unit_source{units.get<part_unit>(), uoff.get<int64_t>() + P, 0, 1},
                                               ceil_div(bound, (int64_t)P), R, grec.get<uint64_t>(), gcap,
                                               flags.get<int>(), orec, ocount, rec_cap, rec_ovf, s, false,
                                               many_units ? ceil_div(n, (int64_t)P) : 0);
@@ -1041,9 +1046,8 @@ void partition_groupby(const col& key_in, const agg_plan& p, gx_groupby_hint* hi
                                                                           rec_ovf);
         GX_LAUNCHED();
         int fl[8];
-        GX_CUDA(cudaMemcpyAsync(fl, flags.get(), sizeof(fl), cudaMemcpyDeviceToHost, s));
-        if (tail_later) GX_CUDA(cudaMemcpyAsync(tail, uoff.get<int64_t>() + P, sizeof(tail), cudaMemcpyDeviceToHost, s));
-        GX_CUDA(cudaStreamSynchronize(s));
+        host_read(fl, flags.get(), sizeof(fl), s);
+        if (tail_later) host_read(tail, uoff.get<int64_t>() + P, sizeof(tail), s);
         if (tail_later && (int)tail[1])
             fail(GX_ETIMEOUT, "partition scatter: a bulk copy into shared memory did not complete");
         if (fl[1]) { gcap *= 8; continue; }

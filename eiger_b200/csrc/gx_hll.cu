@@ -11,6 +11,7 @@
 // fmix64 of the canonical key bits) makes the large-range correction
 // unnecessary.  Each CTA keeps its registers in shared memory and merges
 // them into the global sketch with one atomicMax per non-zero register.
+#include <algorithm>
 #include <cmath>
 
 #include "gx_groupby.h"
@@ -103,6 +104,18 @@ __global__ void __launch_bounds__(HLLV_NT) k_hll_vec(const void* __restrict__ ke
         if (sreg[i]) atomicMax(&regs[i], sreg[i]);
 }
 
+// Registers of each rank, so that the host reads 64 counts instead of 2^13
+// registers.
+constexpr int HLL_RANKS = 64;
+__global__ void __launch_bounds__(1024) k_hll_ranks(const unsigned* __restrict__ regs, unsigned* __restrict__ out) {
+    __shared__ unsigned c[HLL_RANKS];
+    if (threadIdx.x < HLL_RANKS) c[threadIdx.x] = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < HLL_M; i += 1024) atomicAdd(&c[min(regs[i], HLL_RANKS - 1u)], 1u);
+    __syncthreads();
+    if (threadIdx.x < HLL_RANKS) out[threadIdx.x] = c[threadIdx.x];
+}
+
 template <int KW>
 __global__ void k_minmax(const void* __restrict__ keys, int64_t n, int kind, unsigned long long* out) {
     // Track the order-preserving image; convert back on the host.
@@ -127,18 +140,21 @@ __global__ void k_minmax(const void* __restrict__ keys, int64_t n, int kind, uns
 
 }  // namespace
 
-double hll_estimate(const unsigned* regs) {
-    double m = HLL_M;
-    double alpha = 0.7213 / (1.0 + 1.079 / m);
+// ranks[r]: registers of rank r.  Ranks are at most 64 - HLL_P + 1 = 52, so the
+// sum of the registers' 2^-rank is taken exactly rank by rank.
+static double hll_from_ranks(const unsigned (&ranks)[HLL_RANKS]) {
+    const double m = HLL_M;
+    const double alpha = 0.7213 / (1.0 + 1.079 / m);
     double sum = 0.0;
-    int zeros = 0;
-    for (int i = 0; i < HLL_M; ++i) {
-        sum += std::ldexp(1.0, -(int)regs[i]);
-        zeros += regs[i] == 0;
-    }
+    for (int r = 0; r < HLL_RANKS; ++r) sum += std::ldexp((double)ranks[r], -r);
     double e = alpha * m * m / sum;
-    if (e <= 2.5 * m && zeros > 0) e = m * std::log(m / (double)zeros);
+    if (e <= 2.5 * m && ranks[0] > 0) e = m * std::log(m / (double)ranks[0]);
     return e;
+}
+double hll_estimate(const unsigned* regs) {
+    unsigned ranks[HLL_RANKS] = {};
+    for (int i = 0; i < HLL_M; ++i) ++ranks[std::min<unsigned>(regs[i], HLL_RANKS - 1)];
+    return hll_from_ranks(ranks);
 }
 
 // Registers of the sketch over rows 0, stride, 2*stride, ... (n rows taken).
@@ -171,12 +187,14 @@ void hll_registers(const col& key_in, int64_t n, int64_t stride, unsigned* d_reg
 
 int64_t ndv_estimate(const col& key, cudaStream_t s) {
     if (key.n == 0) return 0;
-    dbuf regs(HLL_M * sizeof(unsigned), s);
+    dbuf regs((HLL_M + HLL_RANKS) * sizeof(unsigned), s);
+    unsigned* ranks = regs.get<unsigned>() + HLL_M;
     hll_registers(key, key.n, 1, regs.get<unsigned>(), s);
-    std::vector<unsigned> h(HLL_M);
-    GX_CUDA(cudaMemcpyAsync(h.data(), regs.get(), HLL_M * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-    GX_CUDA(cudaStreamSynchronize(s));
-    return (int64_t)std::llround(hll_estimate(h.data()));
+    k_hll_ranks<<<1, 1024, 0, s>>>(regs.get<unsigned>(), ranks);
+    GX_LAUNCHED();
+    unsigned h[HLL_RANKS];
+    host_read(h, ranks, sizeof(h), s);
+    return (int64_t)std::llround(hll_from_ranks(h));
 }
 
 void compute_min_max(const col& key, void* min_out, void* max_out, cudaStream_t s) {
@@ -199,8 +217,7 @@ void compute_min_max(const col& key, void* min_out, void* max_out, cudaStream_t 
     else k_minmax<8><<<g, 256, 0, s>>>(k.data, k.n, kind, out.get<unsigned long long>());
     GX_LAUNCHED();
     uint64_t h[2];
-    GX_CUDA(cudaMemcpyAsync(h, out.get(), 16, cudaMemcpyDeviceToHost, s));
-    GX_CUDA(cudaStreamSynchronize(s));
+    host_read(h, out.get(), 16, s);
     // Invert the order-preserving image, widen to int64 / uint64 / double.
     for (int j = 0; j < 2; ++j) {
         uint64_t img = h[j], raw;

@@ -777,8 +777,7 @@ static bool dense_join(const join_inputs& in, const gx_join_hint& hint, bool row
             GX_LAUNCHED();
         }
         int64_t hs[2];
-        GX_CUDA(cudaMemcpyAsync(hs, scal.get(), 16, cudaMemcpyDeviceToHost, s));
-        GX_CUDA(cudaStreamSynchronize(s));
+        host_read(hs, scal.get(), 16, s);
         if ((int)hs[1] == 0) {
             const int64_t total = hs[0];
             if (hint.max_out > 0 && total > hint.max_out)
@@ -872,8 +871,7 @@ bool unique_hash_join(const join_inputs& in, const gx_join_hint& hint, bool rowi
             GX_LAUNCHED();
         }
         int64_t hs[2];
-        GX_CUDA(cudaMemcpyAsync(hs, total_out, 16, cudaMemcpyDeviceToHost, s));
-        GX_CUDA(cudaStreamSynchronize(s));
+        host_read(hs, total_out, 16, s);
         if ((int)hs[1]) {  // a look-back wait gave up
             out->cols.clear();
             return false;
@@ -977,8 +975,7 @@ static void join_core(const join_inputs& in, const gx_join_hint& hint, bool rowi
             GX_LAUNCHED();
         }
         int64_t hs[2];
-        GX_CUDA(cudaMemcpyAsync(hs, scal.get(), 16, cudaMemcpyDeviceToHost, s));
-        GX_CUDA(cudaStreamSynchronize(s));
+        host_read(hs, scal.get(), 16, s);
         if ((int)hs[1] == 0) {
             const int64_t total = hs[0];
             if (hint.max_out > 0 && total > hint.max_out)

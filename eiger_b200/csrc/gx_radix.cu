@@ -879,8 +879,7 @@ void key_image_range(const col& keys, uint64_t* lo, uint64_t* hi, cudaStream_t s
         GX_LAUNCHED();
     }
     uint64_t h[2];
-    GX_CUDA(cudaMemcpyAsync(h, out.get(), 16, cudaMemcpyDeviceToHost, s));
-    GX_CUDA(cudaStreamSynchronize(s));
+    host_read(h, out.get(), 16, s);
     *lo = h[0];
     *hi = h[1];
 }

@@ -154,6 +154,25 @@ void* thread_scratch(int slot, size_t bytes) {
     return x.p;
 }
 
+namespace {
+// Pinned staging of host_read: one small buffer per host thread, freed with it.
+struct pinned_stage {
+    void* p = nullptr;
+    ~pinned_stage() {
+        if (p) cudaFreeHost(p);  // errors ignored: the context may already be gone at exit
+    }
+};
+thread_local pinned_stage t_stage;
+}  // namespace
+
+void host_read(void* dst, const void* dptr, size_t bytes, cudaStream_t s) {
+    require(bytes <= HOST_READ_MAX, "host_read: too many bytes");
+    if (!t_stage.p) GX_CUDA(cudaHostAlloc(&t_stage.p, HOST_READ_MAX, cudaHostAllocPortable));
+    GX_CUDA(cudaMemcpyAsync(t_stage.p, dptr, bytes, cudaMemcpyDeviceToHost, s));
+    GX_CUDA(cudaStreamSynchronize(s));
+    std::memcpy(dst, t_stage.p, bytes);
+}
+
 void pool_free(void* p, cudaStream_t s) {
     if (!p) return;
     size_t n = 0;
