@@ -72,12 +72,12 @@ def test_argsort_and_sort_column(n):
     assert np.array_equal(only.cpu().numpy(), ek)
 
 
-@pytest.mark.parametrize("n", [2, 8191, 8192, 8193, 2048 * 7, 2048 * 7 + 1, (1 << 19) - 1, 1 << 19, 5120 * 149 + 3])
+@pytest.mark.parametrize("n", [2, 61, 255, 256, 257, 8191, 8192, 8193, 2048 * 7, 2048 * 7 + 1, (1 << 19) - 1, 1 << 19, 5120 * 149 + 3])
 @pytest.mark.parametrize("kdt,vdt", [(np.int8, np.int64), (np.uint16, np.int32), (np.int32, np.int32),
                                      (np.float32, np.int64), (np.int64, np.int64), (np.float64, np.int32)])
 def test_sort_one_cta_and_onesweep_edges(n, kdt, vdt):
-    # The one-CTA sort (up to 8192 rows) and the look-back passes at the edges
-    # of their tiles, from views that start on and off 16-byte boundaries, with
+    # The counting sort (up to 256 rows), the one-CTA sort (up to 8192) and the
+    # look-back passes at the edges of their tiles, from views that start on and off 16-byte boundaries, with
     # keys whose digits vary, are all the same in some passes (skipped) or in
     # all of them, as pairs and as row ids.
     rng = np.random.default_rng(n)
