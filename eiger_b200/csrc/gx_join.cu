@@ -17,6 +17,9 @@
 //      count kernel sizes every tile's output exactly, an exclusive scan
 //      places the tiles, and a write kernel emits every (build, probe) pair
 //      in probe order — deterministic, no wrap, no atomics.
+// Unique build keys, the common dimension table, need no sort: dense ones are
+// placed by key (dense_join), other integers go into a hash table
+// (unique_hash_join); both probe once and place tiles by a look-back.
 // GX_JOIN_SORT_MERGE sorts the probe side too (key + row id) and runs the
 // same matcher over the sorted stream: the reference's sort-both-sides
 // structure, kept for comparison.
@@ -332,17 +335,21 @@ __global__ void __launch_bounds__(JP_NT) k_dense_write(const void* __restrict__ 
 // Look-back", NVIDIA TR 2016).  Probe keys are read and looked up once
 // instead of twice.  Every wait is bounded: a tile that gives up sets *err,
 // publishes anyway so its successors do not wait on it, and writes nothing;
-// the host then reruns the two-pass probe.
+// the host then reruns the two-pass probe.  (A successor that has not seen
+// *err yet writes inside its buffers, which the host drops.)
 // ---------------------------------------------------------------------------
 constexpr unsigned long long TS_AGG = 1ull << 62, TS_INC = 2ull << 62, TS_VAL = (1ull << 62) - 1;
 constexpr int LOOKBACK_SPIN_LIMIT = 1 << 20;
 
-__device__ __forceinline__ void st_release_u64(unsigned long long* p, unsigned long long v) {
-    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+// A state word holds its flag and value together, and nothing else is read on
+// its strength, so relaxed accesses do: the look-back chain bounds the rate of
+// tiles, and an acquire load or a release store lengthens every link of it.
+__device__ __forceinline__ void st_state(unsigned long long* p, unsigned long long v) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
-__device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long* p) {
+__device__ __forceinline__ unsigned long long ld_state(const unsigned long long* p) {
     unsigned long long v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
 
@@ -350,15 +357,15 @@ __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long
 __device__ __forceinline__ int64_t lookback(unsigned long long* tstate, int64_t tile, int64_t total, int* err) {
     const int lane = threadIdx.x & 31;
     if (tile == 0) {
-        if (lane == 0) st_release_u64(tstate, TS_INC | (unsigned long long)total);
+        if (lane == 0) st_state(tstate, TS_INC | (unsigned long long)total);
         return 0;
     }
-    if (lane == 0) st_release_u64(tstate + tile, TS_AGG | (unsigned long long)total);
+    if (lane == 0) st_state(tstate + tile, TS_AGG | (unsigned long long)total);
     int64_t excl = 0, end = tile - 1;  // lane j looks at tile end - j
     int spins = 0;
     while (true) {
         int64_t j = end - lane;
-        unsigned long long st = j >= 0 ? ld_acquire_u64(tstate + j) : TS_INC;
+        unsigned long long st = j >= 0 ? ld_state(tstate + j) : TS_INC;
         unsigned inc = __ballot_sync(0xffffffffu, (st >> 62) == 2);
         unsigned none = __ballot_sync(0xffffffffu, (st >> 62) == 0);
         int stop = inc ? __ffs(inc) - 1 : 31;  // nearest inclusive predecessor, else the whole window
@@ -376,7 +383,7 @@ __device__ __forceinline__ int64_t lookback(unsigned long long* tstate, int64_t 
         if (inc) break;
         end -= 32;
     }
-    if (lane == 0) st_release_u64(tstate + tile, TS_INC | (unsigned long long)(excl + total));
+    if (lane == 0) st_state(tstate + tile, TS_INC | (unsigned long long)(excl + total));
     return excl;
 }
 
@@ -407,7 +414,7 @@ __global__ void __launch_bounds__(JP_NT) k_dense_probe1(const void* __restrict__
     int64_t wbase = dev_::block_exclusive_sum<JP_NT, int64_t>(lane == 0 ? wtot : 0, sm, &total);
     if (warp == 0) {
         int64_t excl = lookback(tstate, tile, total, err);
-        __syncwarp();  // orders the lanes' acquire loads before lane 0 reads the error flag
+        __syncwarp();
         if (lane == 0) {
             s_excl = excl;
             s_skip = *(volatile int*)err;
@@ -483,7 +490,7 @@ __global__ void __launch_bounds__(JP_NT) k_sorted_probe1(build_run b, probe_side
     int64_t wbase = dev_::block_exclusive_sum<JP_NT, int64_t>(lane == 0 ? wtot : 0, sm, &total);
     if (warp == 0) {
         const int64_t excl = lookback(tstate, tile, total, err);
-        __syncwarp();  // orders the lanes' acquire loads before lane 0 reads the error flag
+        __syncwarp();
         if (lane == 0) {
             s_excl = excl;
             s_skip = *(volatile int*)err;
@@ -531,7 +538,7 @@ __global__ void __launch_bounds__(JP_NT) k_sorted_probe1(build_run b, probe_side
 // for 4-byte keys whose output needs the build row; else 16 bytes (key, the
 // one payload or the row).  Rows come out in probe order, as from the sorted
 // run.  10^6 sparse int64 keys and payloads joined to 3 * 10^7 rows with
-// payloads: 1.05 ms a call, 1.55 ms through the sorted run.
+// payloads: 0.99 ms a call, 1.55 ms through the sorted run.
 // Duplicated build keys, and an 8-byte key equal to the empty marker, set
 // *bad; the caller then takes its other plan.
 // ---------------------------------------------------------------------------
@@ -563,7 +570,7 @@ __global__ void __launch_bounds__(UH_NT) k_uniq_build(const void* __restrict__ k
         if (KW == 4) k = __ldg(static_cast<const unsigned*>(keys) + i);
         else k = __ldg(static_cast<const unsigned long long*>(keys) + i);
         if (KW == 8 && k == UH_EMPTY8K) { atomicExch(bad, 1); return; }
-        uint64_t slot = uh_hash<KW>(k) & mask;
+        uint64_t slot = uh_hash<KW>(k) & mask & ~uint64_t(1);
         for (;;) {  // ends: the table is at most half full
             if constexpr (SW == 8) {
                 const unsigned long long old = atomicCAS(table + slot, UH_EMPTY8, k << 32 | (unsigned)i);
@@ -610,49 +617,59 @@ __global__ void __launch_bounds__(UH_NT, SW == 8 ? 4 : 3) k_uniq_probe(const uns
         const int64_t i = row0 + k * 32;
         key[k] = i < np ? __ldcs(static_cast<const kt*>(pkeys) + i) : kt(0);
         val[k] = 0;
-        slot[k] = (unsigned)(uh_hash<KW>(key[k]) & mask);
+        slot[k] = (unsigned)(uh_hash<KW>(key[k]) & mask & ~uint64_t(1));
         if (i < np && !(KW == 8 && key[k] == (kt)UH_EMPTY8K)) open |= 1u << k;
     }
-    // Each round reads the next slot of every unresolved row at once; the
-    // table is at most half full, so every walk meets an empty slot.
+    // Each round reads the keys of the next slot pair (one sector) of every
+    // unresolved row at once; the table is at most half full, so every walk
+    // meets an empty slot.  The second slot of a pair is only filled after the
+    // first, so an empty first slot ends a walk too.
+    constexpr unsigned long long EMPTY = SW == 8 ? UH_EMPTY8 : KW == 4 ? UH_EMPTY4K : UH_EMPTY8K;
     while (open) {
-        unsigned long long w[UH_IPT], v[UH_IPT];
+        unsigned long long w0[UH_IPT], w1[UH_IPT];
 #pragma unroll
         for (int k = 0; k < UH_IPT; ++k) {
             if (!((open >> k) & 1u)) continue;
-            if constexpr (SW == 8) w[k] = __ldg(table + slot[k]);
-            else {
-                const ulonglong2 p = __ldg(reinterpret_cast<const ulonglong2*>(table) + slot[k]);
-                w[k] = p.x;
-                v[k] = p.y;
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < UH_IPT; ++k) {
-            if (!((open >> k) & 1u)) continue;
-            bool empty, same;
             if constexpr (SW == 8) {
-                empty = w[k] == UH_EMPTY8;
-                same = (unsigned)(w[k] >> 32) == (unsigned)key[k];
+                const ulonglong2 p = __ldg(reinterpret_cast<const ulonglong2*>(table + slot[k]));
+                w0[k] = p.x;
+                w1[k] = p.y;
             } else {
-                empty = w[k] == uh_empty<KW>();
-                same = w[k] == (unsigned long long)key[k];
+                w0[k] = __ldg(table + 2 * (uint64_t)slot[k]);
+                w1[k] = __ldg(table + 2 * (uint64_t)slot[k] + 2);
             }
-            if (empty || same) open &= ~(1u << k);
-            if (!empty && same) {
-                hit |= 1u << k;
-                if constexpr (SW == 8) val[k] = (unsigned)w[k];
-                else val[k] = v[k];
-            }
-            slot[k] = (slot[k] + 1) & (unsigned)mask;
         }
+#pragma unroll
+        for (int k = 0; k < UH_IPT; ++k) {
+            if (!((open >> k) & 1u)) continue;
+            auto same = [&](unsigned long long w) {
+                return w != EMPTY && (SW == 8 ? (unsigned)(w >> 32) == (unsigned)key[k] : w == (unsigned long long)key[k]);
+            };
+            if (same(w0[k])) {
+                hit |= 1u << k;
+                if constexpr (SW == 8) val[k] = (unsigned)w0[k];
+            } else if (same(w1[k])) {
+                hit |= 1u << k;
+                if constexpr (SW == 8) val[k] = (unsigned)w1[k];
+                else slot[k] += 1;
+            } else if (w0[k] != EMPTY && w1[k] != EMPTY) {
+                slot[k] = (slot[k] + 2) & (unsigned)mask;
+                continue;
+            }
+            open &= ~(1u << k);
+        }
+    }
+    if constexpr (SW == 16) {
+#pragma unroll
+        for (int k = 0; k < UH_IPT; ++k)
+            if ((hit >> k) & 1u) val[k] = __ldg(table + 2 * (uint64_t)slot[k] + 1);
     }
     const int64_t wtot = dev_::warp_sum((int64_t)__popc(hit));
     int64_t total;
     int64_t wbase = dev_::block_exclusive_sum<UH_NT, int64_t>(lane == 0 ? wtot : 0, sm, &total);
     if (warp == 0) {
         const int64_t excl = lookback(tstate, tile, total, err);
-        __syncwarp();  // orders the lanes' acquire loads before lane 0 reads the error flag
+        __syncwarp();
         if (lane == 0) {
             s_excl = excl;
             s_skip = *(volatile int*)err;
@@ -835,7 +852,7 @@ bool unique_hash_join(const join_inputs& in, const gx_join_hint& hint, bool rowi
     if (nb <= 0 || np <= 0 || nb >= (int64_t)1 << 30 || vkind_of(in.lkey.type) == VK_F || (kw != 4 && kw != 8)) return false;
     const bool pay_in_run = !rowids_only && bpay.size() == 1 && size_of(bpay[0].type) >= 4;
     const int sw = kw == 4 && !pay_in_run ? 8 : 16;
-    const uint64_t cap = next_pow2((uint64_t)nb * 2);
+    const uint64_t cap = next_pow2(std::max<uint64_t>((uint64_t)nb * 2, 4));
     const int64_t ntiles = ceil_div(np, UH_TILE);
     const size_t table_bytes = (size_t)cap * sw;
     try {
