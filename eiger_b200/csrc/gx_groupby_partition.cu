@@ -1112,20 +1112,40 @@ void hash_partition_rows(const col& key, int R, void* keys_out, int64_t* rows_ou
 }
 
 namespace {
+// A warp takes 32 * STARTS_B consecutive rows with their loads in flight
+// together; each row's predecessor comes from the lane before.
+constexpr int STARTS_B = 8;
 template <int KW>
-__global__ void k_part_starts(const void* __restrict__ keys, int64_t n, int kind, int R, int64_t* __restrict__ ps, int P) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i <= n; i += (int64_t)gridDim.x * blockDim.x) {
-        int cur = i < n ? (int)(part_hash<KW>(ld_key<KW>(keys, i, kind)) & (P - 1)) : P;
-        int prev = i > 0 ? (int)(part_hash<KW>(ld_key<KW>(keys, i - 1, kind)) & (P - 1)) : -1;
-        for (int p = prev + 1; p <= cur; ++p) ps[p] = i;
+__global__ void __launch_bounds__(256) k_part_starts(const void* __restrict__ keys, int64_t n, int kind, int R,
+                                                     int64_t* __restrict__ ps, int P) {
+    const int lane = threadIdx.x & 31;
+    const int64_t w = blockIdx.x * (int64_t)(256 / 32) + (threadIdx.x >> 5);
+    const int64_t i0 = w * 32 * STARTS_B;
+    if (i0 > n) return;
+    auto part = [&](int64_t i) { return (int)(part_hash<KW>(ld_key<KW>(keys, i, kind)) & (unsigned)(P - 1)); };
+    int id[STARTS_B];
+#pragma unroll
+    for (int q = 0; q < STARTS_B; ++q) {
+        const int64_t i = i0 + q * 32 + lane;
+        id[q] = i < n ? part(i) : P;  // row n ends the last partition
+    }
+    int last = i0 > 0 ? part(i0 - 1) : -1;  // the row before the next 32
+#pragma unroll
+    for (int q = 0; q < STARTS_B; ++q) {
+        const int64_t i = i0 + q * 32 + lane;
+        int prev = __shfl_up_sync(0xffffffffu, id[q], 1);
+        if (lane == 0) prev = last;
+        last = __shfl_sync(0xffffffffu, id[q], 31);
+        if (i <= n)
+            for (int p = prev + 1; p <= id[q]; ++p) ps[p] = i;
     }
 }
 }  // namespace
 
 void partition_starts(const void* keys, int kw, int64_t n, int kind, int R, int64_t* ps, cudaStream_t s) {
     int P = 1 << R;
-    if (kw == 4) k_part_starts<4><<<grid_for(n + 1, 256, 8), 256, 0, s>>>(keys, n, kind, R, ps, P);
-    else k_part_starts<8><<<grid_for(n + 1, 256, 8), 256, 0, s>>>(keys, n, kind, R, ps, P);
+    if (kw == 4) k_part_starts<4><<<(unsigned)ceil_div(n + 1, 256 * STARTS_B), 256, 0, s>>>(keys, n, kind, R, ps, P);
+    else k_part_starts<8><<<(unsigned)ceil_div(n + 1, 256 * STARTS_B), 256, 0, s>>>(keys, n, kind, R, ps, P);
     GX_LAUNCHED();
 }
 
