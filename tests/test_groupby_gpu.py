@@ -412,7 +412,7 @@ def test_partition_groups_per_partition_override(monkeypatch):
     assert_columns_match(got, exp)
 
 
-@pytest.mark.parametrize("n", [70_001, 4096 * 37 + 5, 300_000])
+@pytest.mark.parametrize("n", [70_001, 2048 * 40, 4096 * 37 + 5, 300_000])
 @pytest.mark.parametrize("kdt", [np.int32, np.int64])
 @pytest.mark.parametrize("skew", [False, True])
 def test_partition_two_passes_small_units(n, kdt, skew):
@@ -431,3 +431,27 @@ def test_partition_two_passes_small_units(n, kdt, skew):
                                [(0, O.SUM), (0, O.MIN), (1, O.SUM), (1, O.MAX)])):
         t = gx.groupby([to_dev(key)], [to_dev(v) for v in vals], reqs, gx.make_hint(gx.PARTITION, radix_bits=10))
         assert_columns_match(sort_by_key(t.numpy_columns()), list(O.groupby(key, vals, oreqs)))
+
+
+@pytest.mark.parametrize("algo", [gx.HASH, gx.PARTITION])
+@pytest.mark.parametrize("kdt", [np.int32, np.int64])
+@pytest.mark.parametrize("share,G", [(0.97, 700), (0.6, 3000), (1.0, 1), (0.3, 300)])
+def test_heavy_key_in_split_units(algo, kdt, share, G):
+    # Pieces of a partition that one key has most of: its rows are updated
+    # together (folded float sums, read-first MIN and MAX), the others by
+    # themselves; zeros of both signs and infinities among the values.
+    n = 600_011
+    rng = np.random.default_rng(G)
+    key = rng.integers(0, G, n).astype(kdt) * kdt(1009) - kdt(7)
+    key[rng.random(n) < share] = kdt(-7)
+    iv = rng.integers(-2**62, 2**62, n)
+    fv = rng.choice(np.array([0.0, -0.0, 1.5, -2.25, 1e300, 3e-310]), n) * rng.choice(np.array([1.0, 0.5]), n)
+    gv = np.where(rng.random(n) < 1e-4, np.inf, rng.random(n))
+    for f in (fv, gv):
+        ops = [(0, "SUM"), (0, "MIN"), (0, "MAX"), (1, "SUM"), (1, "MIN"), (1, "MAX"), (0, "COUNT_ALL")]
+        t = gx.groupby([to_dev(key)], [to_dev(iv), to_dev(f)], [(c, getattr(gx, o)) for c, o in ops],
+                       gx.make_hint(algo, G, radix_bits=1 if algo == gx.PARTITION else 0))
+        exp = O.groupby(key, [iv, f], [(c, getattr(O, o)) for c, o in ops])
+        # Sums in another order: at most n roundings of the sum of magnitudes.
+        bound = n * 2.0**-53 * max(1.0, float(np.abs(f[np.isfinite(f)]).sum() / max(1e-300, abs(f[np.isfinite(f)].sum()))))
+        assert_columns_match(sort_by_key(t.numpy_columns()), list(exp), float_cols_rtol=max(1e-12, bound))
