@@ -367,7 +367,6 @@ inline int grid_for(int64_t work_items, int per_block, int blocks_per_sm = 4) {
 
 // Fill a device buffer of 8-byte words with a pattern (kernel in gx_util.cu).
 void fill_u64(void* dst, uint64_t pattern, int64_t words, cudaStream_t s);
-void fill_u32(void* dst, uint32_t pattern, int64_t words, cudaStream_t s);
 // Exclusive scan of int64 counts into offsets (n+1 outputs, out[n] = total).
 void exclusive_scan_i64(const int64_t* in, int64_t* out, int64_t n, cudaStream_t s);
 // The same scan with its temporaries carved from caller scratch.

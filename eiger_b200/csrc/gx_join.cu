@@ -748,6 +748,10 @@ join_out make_outputs(const join_inputs& in, bool build_left, bool rowids_only, 
     return o;
 }
 
+// Probe rows up to which a probe is queued before the build's flag is read:
+// its wait costs a small join about as much as the probe does.
+constexpr int64_t PROBE_AHEAD = 1 << 20;
+
 // Returns false when the build keys turn out not to be unique.
 static bool dense_join(const join_inputs& in, const gx_join_hint& hint, bool rowids_only, bool build_left,
                        uint64_t lo, uint64_t hi, cudaStream_t s, gx_table* out) {
@@ -757,35 +761,42 @@ static bool dense_join(const join_inputs& in, const gx_join_hint& hint, bool row
     const int kind = vkind_of(in.lkey.type);
     const int64_t nb = bkey.n, np = pkey.n;
     uint64_t npos = hi - lo + 1;
-    dbuf slot_row((size_t)npos * 4, s), flag(8, s);
-    fill_u32(slot_row.get(), NO_ROW, (int64_t)npos, s);
-    GX_CUDA(cudaMemsetAsync(flag.get(), 0, 8, s));
+    const int64_t ntiles = ceil_div(std::max<int64_t>(np, 1), JP_TILE);
+    // Tile states, then ticket, total, look-back error and duplicate flag (16
+    // bytes of total and flags read together).  Apart from the placement array:
+    // one buffer of 64 MB and a little made the stream pool remap the outputs'
+    // gigabytes on every other call (3 -> 21 ms).
+    const size_t ctl_bytes = (size_t)ntiles * 8 + 24;
+    dbuf slots((size_t)npos * 4, s), control(ctl_bytes, s);
+    uint32_t* slot_row = slots.get<uint32_t>();
+    char* ctl = control.get<char>();
+    unsigned long long* tstate = reinterpret_cast<unsigned long long*>(ctl);
+    unsigned* ticket = reinterpret_cast<unsigned*>(ctl + (size_t)ntiles * 8);
+    int64_t* total_out = reinterpret_cast<int64_t*>(ctl + (size_t)ntiles * 8 + 8);
+    int* err = reinterpret_cast<int*>(total_out + 1);
+    int* dup = err + 1;
+    GX_CUDA(cudaMemsetAsync(slot_row, 0xFF, (size_t)npos * 4, s));  // NO_ROW
+    GX_CUDA(cudaMemsetAsync(ctl, 0, ctl_bytes, s));
     {
         GX_PROF("join_build_place", s);
-        if (kw == 4) k_dense_place<4><<<grid_for(nb, 256, 8), 256, 0, s>>>(bkey.data, nb, kind, lo, slot_row.get<uint32_t>(), flag.get<int>());
-        else k_dense_place<8><<<grid_for(nb, 256, 8), 256, 0, s>>>(bkey.data, nb, kind, lo, slot_row.get<uint32_t>(), flag.get<int>());
+        if (kw == 4) k_dense_place<4><<<grid_for(nb, 256, 8), 256, 0, s>>>(bkey.data, nb, kind, lo, slot_row, dup);
+        else k_dense_place<8><<<grid_for(nb, 256, 8), 256, 0, s>>>(bkey.data, nb, kind, lo, slot_row, dup);
         GX_LAUNCHED();
     }
-    if (read_scalar(flag.get<int>(), s)) return false;
-    int64_t ntiles = ceil_div(std::max<int64_t>(np, 1), JP_TILE);
     static const bool two_pass = getenv("GX_JOIN_TWO_PASS") != nullptr;
-    if (np > 0 && !two_pass) {
+    const bool one_pass = np > 0 && !two_pass;
+    // A short probe runs before the duplicate flag is known (each position
+    // holds one row, so it stays inside its outputs) and is dropped with it.
+    if (!(one_pass && np <= PROBE_AHEAD) && read_scalar(dup, s)) return false;
+    if (one_pass) {
         // Unique build keys: at most np matches, so the outputs are allocated
         // up front and the probe runs once.
-        dbuf tstate((size_t)ntiles * 8 + 16, s), scal(16, s);
-        GX_CUDA(cudaMemsetAsync(tstate.get(), 0, (size_t)ntiles * 8 + 16, s));
-        GX_CUDA(cudaMemsetAsync(scal.get(), 0, 16, s));
         join_out o = make_outputs(in, build_left, rowids_only, false, true, np, s, out, np);
-        unsigned* ticket = reinterpret_cast<unsigned*>(tstate.get<char>() + (size_t)ntiles * 8);
-        int64_t* total_out = scal.get<int64_t>();
-        int* err = reinterpret_cast<int*>(scal.get<char>() + 8);
         {
             GX_PROF("join_probe_write", s);
-#define GX_PROBE1(KW_, RID_)                                                                            \
-    k_dense_probe1<KW_, RID_><<<(unsigned)ntiles, JP_NT, 0, s>>>(pkey.data, np, kind, lo, hi,              \
-                                                                 slot_row.get<uint32_t>(),                \
-                                                                 tstate.get<unsigned long long>(), ticket, \
-                                                                 ntiles, total_out, err, o)
+#define GX_PROBE1(KW_, RID_)                                                                                 \
+    k_dense_probe1<KW_, RID_><<<(unsigned)ntiles, JP_NT, 0, s>>>(pkey.data, np, kind, lo, hi, slot_row, tstate, \
+                                                                 ticket, ntiles, total_out, err, o)
             if (kw == 4 && rowids_only) GX_PROBE1(4, true);
             else if (kw == 4) GX_PROBE1(4, false);
             else if (rowids_only) GX_PROBE1(8, true);
@@ -794,7 +805,11 @@ static bool dense_join(const join_inputs& in, const gx_join_hint& hint, bool row
             GX_LAUNCHED();
         }
         int64_t hs[2];
-        host_read(hs, scal.get(), 16, s);
+        host_read(hs, total_out, 16, s);
+        if (hs[1] >> 32) {  // duplicate build keys
+            out->cols.clear();
+            return false;
+        }
         if ((int)hs[1] == 0) {
             const int64_t total = hs[0];
             if (hint.max_out > 0 && total > hint.max_out)
@@ -809,8 +824,8 @@ static bool dense_join(const join_inputs& in, const gx_join_hint& hint, bool row
     int64_t total = 0;
     if (np > 0) {
         GX_PROF("join_probe_count", s);
-        if (kw == 4) k_dense_count<4><<<(unsigned)ntiles, JP_NT, 0, s>>>(pkey.data, np, kind, lo, hi, slot_row.get<uint32_t>(), tc.get<int64_t>());
-        else k_dense_count<8><<<(unsigned)ntiles, JP_NT, 0, s>>>(pkey.data, np, kind, lo, hi, slot_row.get<uint32_t>(), tc.get<int64_t>());
+        if (kw == 4) k_dense_count<4><<<(unsigned)ntiles, JP_NT, 0, s>>>(pkey.data, np, kind, lo, hi, slot_row, tc.get<int64_t>());
+        else k_dense_count<8><<<(unsigned)ntiles, JP_NT, 0, s>>>(pkey.data, np, kind, lo, hi, slot_row, tc.get<int64_t>());
         GX_LAUNCHED();
         exclusive_scan_i64(tc.get<int64_t>(), toff.get<int64_t>(), ntiles, s);
         total = read_scalar(toff.get<int64_t>() + ntiles, s);
@@ -821,8 +836,8 @@ static bool dense_join(const join_inputs& in, const gx_join_hint& hint, bool row
     join_out o = make_outputs(in, build_left, rowids_only, false, true, total, s, out);
     if (total > 0) {
         GX_PROF("join_probe_write", s);
-        if (kw == 4) k_dense_write<4><<<(unsigned)ntiles, JP_NT, 0, s>>>(pkey.data, np, kind, lo, hi, slot_row.get<uint32_t>(), toff.get<int64_t>(), o);
-        else k_dense_write<8><<<(unsigned)ntiles, JP_NT, 0, s>>>(pkey.data, np, kind, lo, hi, slot_row.get<uint32_t>(), toff.get<int64_t>(), o);
+        if (kw == 4) k_dense_write<4><<<(unsigned)ntiles, JP_NT, 0, s>>>(pkey.data, np, kind, lo, hi, slot_row, toff.get<int64_t>(), o);
+        else k_dense_write<8><<<(unsigned)ntiles, JP_NT, 0, s>>>(pkey.data, np, kind, lo, hi, slot_row, toff.get<int64_t>(), o);
         GX_LAUNCHED();
     }
     GX_CUDA(cudaStreamSynchronize(s));
@@ -877,7 +892,7 @@ bool unique_hash_join(const join_inputs& in, const gx_join_hint& hint, bool rowi
             else k_uniq_build<8, 16><<<g, UH_NT, 0, s>>>(bkey.data, pay, pw, nb, tb, cap - 1, bad);
             GX_LAUNCHED();
         }
-        if (read_scalar(bad, s)) return false;
+        if (np > PROBE_AHEAD && read_scalar(bad, s)) return false;
         join_out o = make_outputs(in, build_left, rowids_only, pay_in_run, false, np, s, out, np);
         {
             GX_PROF("join_probe_write", s);
@@ -889,7 +904,7 @@ bool unique_hash_join(const join_inputs& in, const gx_join_hint& hint, bool rowi
         }
         int64_t hs[2];
         host_read(hs, total_out, 16, s);
-        if ((int)hs[1]) {  // a look-back wait gave up
+        if (hs[1]) {  // a look-back wait gave up (low half), or the build flag (high half)
             out->cols.clear();
             return false;
         }

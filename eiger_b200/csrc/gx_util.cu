@@ -213,11 +213,6 @@ __global__ void k_fill_u64(uint64_t* __restrict__ d, uint64_t v, int64_t n) {
     int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (; i < n; i += stride) d[i] = v;
 }
-__global__ void k_fill_u32(uint32_t* __restrict__ d, uint32_t v, int64_t n) {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (; i < n; i += stride) d[i] = v;
-}
 __global__ void k_sequence(int64_t* __restrict__ d, int64_t n, int64_t start, int64_t step) {
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -329,11 +324,6 @@ __global__ void k_set_last(const int64_t* __restrict__ tile_prefix, int64_t ntil
 void fill_u64(void* dst, uint64_t pattern, int64_t words, cudaStream_t s) {
     if (words <= 0) return;
     k_fill_u64<<<grid_for(words, 256, 8), 256, 0, s>>>(static_cast<uint64_t*>(dst), pattern, words);
-    GX_LAUNCHED();
-}
-void fill_u32(void* dst, uint32_t pattern, int64_t words, cudaStream_t s) {
-    if (words <= 0) return;
-    k_fill_u32<<<grid_for(words, 256, 8), 256, 0, s>>>(static_cast<uint32_t*>(dst), pattern, words);
     GX_LAUNCHED();
 }
 void sequence_i64(int64_t* out, int64_t n, int64_t start, int64_t step, cudaStream_t s) {
