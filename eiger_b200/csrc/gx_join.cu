@@ -845,16 +845,21 @@ static bool dense_join(const join_inputs& in, const gx_join_hint& hint, bool row
 }
 
 // Gives back most of outputs that were allocated for `cap` rows and hold far
-// fewer: copied to exact buffers when less than half is used.
+// fewer: copied to exact buffers when less than half is used.  Waits for the
+// copies, since a join returns with its rows written.
 static void shrink_outputs(gx_table* out, int64_t cap, int64_t total, cudaStream_t s) {
+    bool copied = false;
     for (auto& c : out->cols) {
         c.size = total;
         if (total >= cap / 2) continue;
         owned_col e = make_col(c.type, total, s);
-        if (total > 0)
+        if (total > 0) {
             GX_CUDA(cudaMemcpyAsync(e.buf.get(), c.buf.get(), (size_t)total * size_of(c.type), cudaMemcpyDeviceToDevice, s));
+            copied = true;
+        }
         c.buf = std::move(e.buf);
     }
+    if (copied) GX_CUDA(cudaStreamSynchronize(s));
 }
 
 bool unique_hash_join(const join_inputs& in, const gx_join_hint& hint, bool rowids_only, bool build_left,

@@ -159,3 +159,42 @@ def test_unique_sparse_keys_one_pass(algo, kdt, nb, npr):
                     swap = nb > npr
                     assert not swap and np.array_equal(p[o], er[e]) and np.array_equal(b[o], bp[el][e])
                     assert np.array_equal(key[o], pk[er[e]])
+
+
+@pytest.mark.parametrize("algo", [gx.JOIN_SORT, gx.JOIN_HASH])
+@pytest.mark.parametrize("form", ["rowids", "table"])
+@pytest.mark.parametrize("npr,share", [(1 << 20, 0.05), (1 << 24, 0.05), (1 << 24, 0.45)])
+def test_selective_join_is_written_when_it_returns(algo, form, npr, share):
+    # Few matches of sparse unique keys, on a stream that the NULL stream does
+    # not wait for: nothing may be left in flight when the call returns (the
+    # result is read through the NULL stream).
+    import torch
+    nb, step, n_pay = 100_003, 1_000_003, 6
+    g = torch.Generator(device="cuda")
+    g.manual_seed(npr)
+    ids = torch.randperm(nb, device="cuda", generator=g)
+    pid = torch.randint(0, nb, (npr,), device="cuda", generator=g)
+    miss = torch.rand(npr, device="cuda", generator=g) >= share
+    bk, pk = ids * step, (pid + miss * nb) * step
+    row_of = torch.empty_like(ids)
+    row_of[ids] = torch.arange(nb, device="cuda")
+    want_p = torch.nonzero(~miss).squeeze(1)
+    want_b = row_of[pid[want_p]]
+    pays = [pk * (c + 2) for c in range(n_pay)]
+    hint = gx.make_join_hint(algo, gx.MAT_GFUR)
+    s = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for _ in range(3):
+        if form == "rowids":
+            t = gx.inner_eq_join_rowids(bk, pk, hint, stream=s)
+            assert s.query()
+            b, p = t.numpy_columns()
+            assert np.array_equal(b, want_b.cpu().numpy()) and np.array_equal(p, want_p.cpu().numpy())
+        else:
+            t = gx.inner_eq_join([bk, ids], [pk, *pays], hint, stream=s)
+            assert s.query()
+            cols = t.numpy_columns()
+            assert np.array_equal(cols[0], pk[want_p].cpu().numpy()) and np.array_equal(cols[1], pid[want_p].cpu().numpy())
+            for c in range(n_pay):
+                assert np.array_equal(cols[2 + c], pays[c][want_p].cpu().numpy())
+        del t
