@@ -835,10 +835,12 @@ __global__ void __launch_bounds__(NT, NT == HGB_NT ? 1 : 4) k_units_dense(const 
                         const unsigned same = __ballot_sync(0xffffffffu, hit && gid[q] == g0);
                         if (__popc(same) >= max(8, 2 * R)) {
                             hot_update(same, src, my_acc, g0 * R, v[q]);
-                            if (lane == src) {
-                                atomicAdd(&my_counts[g0 * R], (unsigned)__popc(same));
-                                s_hot = 1;
-                            }
+                            // Each replica counts its own rows (one lane adds
+                            // for all of them): one that counts none is left
+                            // out of the merge.
+                            const unsigned mine = same & ((0xFFFFFFFFu / ((1u << R) - 1u)) << rep);
+                            if (mine && lane == __ffs(mine) - 1) atomicAdd(&my_counts[g0 * R], (unsigned)__popc(mine));
+                            if (lane == src) s_hot = 1;
                             hit = hit && gid[q] != g0;
                         }
                     }

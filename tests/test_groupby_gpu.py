@@ -455,3 +455,31 @@ def test_heavy_key_in_split_units(algo, kdt, share, G):
         # Sums in another order: at most n roundings of the sum of magnitudes.
         bound = n * 2.0**-53 * max(1.0, float(np.abs(f[np.isfinite(f)]).sum() / max(1e-300, abs(f[np.isfinite(f)].sum()))))
         assert_columns_match(sort_by_key(t.numpy_columns()), list(exp), float_cols_rtol=max(1e-12, bound))
+
+
+@pytest.mark.parametrize("algo", [gx.HASH, gx.PARTITION])
+@pytest.mark.parametrize("kdt", [np.int32, np.int64])
+@pytest.mark.parametrize("G", [16, 128, 512])
+@pytest.mark.parametrize("run", [64, 1024])
+def test_runs_of_keys_seen_once_before(algo, kdt, G, run):
+    # Each key once, then long runs of one key: a warp's rows are then all of a
+    # key that few of its accumulator replicas have counted a row of yet.  All
+    # replicas' sums and extremes belong to the result.
+    rng = np.random.default_rng(G + run)
+    n = 148 * 7000 + 11
+    blocks, rows = [], 0
+    while rows < n:
+        singles = rng.permutation(G)
+        runs = np.repeat(rng.integers(0, G, max(1, 3072 // run)), run)
+        blocks += [singles, runs]
+        rows += len(singles) + len(runs)
+    key = np.concatenate(blocks)[:n].astype(kdt) * kdt(1009) - kdt(7)
+    iv = rng.integers(-2**62, 2**62, n)
+    fv = rng.random(n) - 0.25
+    ops = [(0, "SUM"), (0, "MIN"), (0, "MAX"), (1, "SUM"), (1, "MIN"), (1, "MAX"), (0, "COUNT_ALL")]
+    t = gx.groupby([to_dev(key)], [to_dev(iv), to_dev(fv)], [(c, getattr(gx, o)) for c, o in ops],
+                   gx.make_hint(algo, G, radix_bits=1 if algo == gx.PARTITION else 0))
+    exp = O.groupby(key, [iv, fv], [(c, getattr(O, o)) for c, o in ops])
+    # Sums in another order: at most n roundings of the sum of magnitudes.
+    bound = n * 2.0**-53 * float(np.abs(fv).sum() / fv.sum())
+    assert_columns_match(sort_by_key(t.numpy_columns()), list(exp), float_cols_rtol=max(1e-12, bound))
