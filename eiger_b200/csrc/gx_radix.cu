@@ -23,6 +23,7 @@
 // state: it serves the allocation-free sort, and a sort whose look-back gave
 // up runs through it again.
 #include <algorithm>
+#include <cstdlib>
 
 #include "gx_groupby.h"
 
@@ -333,7 +334,7 @@ constexpr int OS_MAX_PASSES = 8;
 struct os_plan {
     unsigned long long hist[OS_MAX_PASSES][RS_BINS];
     unsigned long long base[OS_MAX_PASSES][RS_BINS];
-    int order[OS_MAX_PASSES];  // position among the passes that run, -1: skipped
+    int order[OS_MAX_PASSES];  // position among the passes that run, -1: skipped, or one before it gave up
     int runs;                  // passes that run
     unsigned ticket[OS_MAX_PASSES];
     unsigned done;
@@ -486,6 +487,7 @@ struct os_args {
     void *ktmp, *vtmp, *kout, *vout;
     int64_t n;
     int pass, iota;
+    int spin_limit;      // empty polls before a look-back gives up (0: at once)
     os_state* state[2];  // [tile][digit]; the running pass uses one and clears the other
     os_plan* plan;
 };
@@ -522,6 +524,11 @@ constexpr int os_ipt_max() {
 // Two CTAs of 512 threads with 6144 rows beat three of 4608 rows (9.05 against
 // 10.6 ms a sort), one of 1024 threads (9.6 ms) and 768 threads (10.6 ms); a
 // look-back window of 8 tiles beats 4 and 16 by 3% and 10%.
+// A tile whose look-back gives up writes nothing, sets plan->err and takes the
+// later passes off the plan.  So none of them ranks the holes of this pass
+// against digit starts that were counted from all rows, and every position
+// written lies inside its digit's range.  (Reading plan->err at the start of
+// each tile instead cost 1.6% of a sort.)
 template <int KW, int VW, bool FLT, int IPT>
 __global__ void __launch_bounds__(OS_NT, 2) k_radix_onesweep(digit_of<KW, FLT> dg, os_args a) {
     using vt = typename std::conditional<VW == 8, unsigned long long, uint32_t>::type;
@@ -539,7 +546,9 @@ __global__ void __launch_bounds__(OS_NT, 2) k_radix_onesweep(digit_of<KW, FLT> d
     void* kout = (left & 1) ? a.ktmp : a.kout;
     void* vout = (left & 1) ? a.vtmp : a.vout;
     const bool iota = a.iota && ord == 0;
-    os_state* state = a.state[ord & 1];
+    // Selected, not indexed: an index would put the arguments on the stack.
+    os_state* state = ord & 1 ? a.state[1] : a.state[0];
+    os_state* next_state = ord & 1 ? a.state[0] : a.state[1];
 
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     unsigned char* skeys = smem;
@@ -580,7 +589,7 @@ __global__ void __launch_bounds__(OS_NT, 2) k_radix_onesweep(digit_of<KW, FLT> d
     const int64_t tile_base = tile * TILE;
     const int tile_n = (int)min((int64_t)TILE, a.n - tile_base);
     const bool full = tile_n == TILE;
-    if (t < RS_BINS) st_state(a.state[(ord & 1) ^ 1] + tile * RS_BINS + t, 0ull);
+    if (t < RS_BINS) st_state(next_state + tile * RS_BINS + t, 0ull);
     auto row_key = [&](int i) -> kreg<KW> {
         if constexpr (KW == 1) return skeys[i];
         else if constexpr (KW == 2) return reinterpret_cast<const unsigned short*>(skeys)[i];
@@ -653,7 +662,8 @@ __global__ void __launch_bounds__(OS_NT, 2) k_radix_onesweep(digit_of<KW, FLT> d
     if (t < RS_BINS) {
         os_state before = 0;
         int64_t j = tile - 1;
-        for (int spins = 0; j >= 0;) {
+        if (j >= 0 && a.spin_limit == 0) failed = 1;
+        for (int spins = 0; j >= 0 && !failed;) {
             os_state st[OS_WIN];
 #pragma unroll
             for (int q = 0; q < OS_WIN; ++q) st[q] = j - q >= 0 ? ld_state(state + (j - q) * RS_BINS + t) : OS_INC;
@@ -674,7 +684,7 @@ __global__ void __launch_bounds__(OS_NT, 2) k_radix_onesweep(digit_of<KW, FLT> d
             if (inc || failed) break;
             j -= seen;
             if (seen == 0) {
-                if (++spins > OS_SPIN_LIMIT) { failed = 1; break; }
+                if (++spins > a.spin_limit) { failed = 1; break; }
                 __nanosleep(20);
             }
         }
@@ -685,6 +695,7 @@ __global__ void __launch_bounds__(OS_NT, 2) k_radix_onesweep(digit_of<KW, FLT> d
     if (__syncthreads_or(failed)) {
         if (t == 0) {
             atomicExch(&a.plan->err, 1);
+            for (int p = a.pass + 1; p < OS_MAX_PASSES; ++p) a.plan->order[p] = -1;
             // Leave no copy in flight into this CTA's shared memory.
             if (full && kbulk) dev_::mbar_wait_bounded(bar0, 0, OS_COPY_WAIT);
             if (full && load_vals && vbulk) dev_::mbar_wait_bounded(bar1, 0, OS_COPY_WAIT);
@@ -851,6 +862,12 @@ size_t onesweep_temp_bytes(int64_t n, int kw, int vw) {
                sizeof(os_state);
 }
 
+// A wait's limit, or the shorter one that a test sets to make it run out.
+int poll_limit(const char* name, int limit) {
+    const char* e = getenv(name);
+    return e ? std::min(std::max(atoi(e), 0), limit) : limit;
+}
+
 // n > 0, begin_bit < end_bit.  Returns false when a look-back wait gave up
 // (the outputs are then unspecified, the inputs untouched).
 template <int KW, int VW, bool FLT>
@@ -897,6 +914,7 @@ bool onesweep_run(const col& keys, const void* vin, bool iota, const img_params&
     tp += r256((size_t)n * VW);
     a.n = n;
     a.iota = iota ? 1 : 0;
+    a.spin_limit = poll_limit("GX_RADIX_LOOKBACK_POLLS", OS_SPIN_LIMIT);
     a.plan = reinterpret_cast<os_plan*>(tp);
     tp += r256(sizeof(os_plan));
     a.state[0] = reinterpret_cast<os_state*>(tp);

@@ -104,6 +104,43 @@ def test_sort_one_cta_and_onesweep_edges(n, kdt, vdt):
         assert np.array_equal(idx.cpu().numpy(), ei)
 
 
+@pytest.mark.parametrize("n", [50_000, 512 * 4 * 300 + 7, 4608 * 148 * 5 + 1])
+@pytest.mark.parametrize("kdt,vdt", [(np.int32, np.int64), (np.float64, np.int32), (np.int64, np.int64)])
+@pytest.mark.parametrize("off", [0, 1])
+def test_sort_whose_look_back_gives_up(monkeypatch, n, kdt, vdt, off):
+    # Every tile but the first gives up at once (limit 0), or where the tile
+    # before it is late (limit 1): the passes that follow move nothing and the
+    # per-tile passes sort the untouched inputs.
+    rng = np.random.default_rng(n)
+    key = rng.integers(0, 256, size=(n + 1) * np.dtype(kdt).itemsize, dtype=np.uint8).view(kdt)
+    if np.dtype(kdt).kind == "f":
+        key = (rng.integers(-10**6, 10**6, n + 1) / 8).astype(kdt)
+    val = np.arange(n + 1).astype(vdt)
+    dk, dv = to_dev(key), to_dev(val)
+    ek, ev = O.sort_pairs(key[off:off + n].copy(), val[off:off + n].copy(), 0, -1, False)
+
+    def launches_of_a_sort():
+        ko, vo = gx.OwnedColumn(), gx.OwnedColumn()
+        before = gx.kernel_launches()
+        gx.check(gx.lib.gx_sort_column_pair(
+            gx.ColumnView(dk.data_ptr(), n, gx._NP_TO_GX[np.dtype(kdt)], off),
+            gx.ColumnView(dv.data_ptr(), n, gx._NP_TO_GX[np.dtype(vdt)], off), 0, -1, 0, None, 0,
+            gx._stream_ptr(None), C.byref(ko), C.byref(vo)))
+        used = gx.kernel_launches() - before
+        assert np.array_equal(gx.owned_to_torch(ko).cpu().numpy().view(np.uint8), ek.view(np.uint8))
+        assert np.array_equal(gx.owned_to_torch(vo).cpu().numpy(), ev)
+        return used
+
+    plain = launches_of_a_sort()
+    monkeypatch.setenv("GX_RADIX_LOOKBACK_POLLS", "0")
+    assert launches_of_a_sort() > plain  # the one-sweep passes and the per-tile ones
+    monkeypatch.setenv("GX_RADIX_LOOKBACK_POLLS", "1")
+    launches_of_a_sort()
+    assert np.array_equal(dk.cpu().numpy().view(np.uint8), key.view(np.uint8))
+    monkeypatch.delenv("GX_RADIX_LOOKBACK_POLLS")
+    assert launches_of_a_sort() == plain
+
+
 @pytest.mark.parametrize("kdt", [np.int32, np.int64])
 def test_partition_and_offsets_reference_case(kdt):
     # sort_partition_test.cu:16-59 shapes (4864 / 4865 rows, bits 0..5).
