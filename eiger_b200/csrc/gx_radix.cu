@@ -488,6 +488,7 @@ struct os_args {
     int64_t n;
     int pass, iota;
     int spin_limit;      // empty polls before a look-back gives up (0: at once)
+    uint32_t copy_limit; // polls of a copy
     os_state* state[2];  // [tile][digit]; the running pass uses one and clears the other
     os_plan* plan;
 };
@@ -524,8 +525,9 @@ constexpr int os_ipt_max() {
 // Two CTAs of 512 threads with 6144 rows beat three of 4608 rows (9.05 against
 // 10.6 ms a sort), one of 1024 threads (9.6 ms) and 768 threads (10.6 ms); a
 // look-back window of 8 tiles beats 4 and 16 by 3% and 10%.
-// A tile whose look-back gives up writes nothing, sets plan->err and takes the
-// later passes off the plan.  So none of them ranks the holes of this pass
+// A tile whose look-back gives up, or whose rows did not arrive, writes nothing,
+// sets plan->err and takes the later passes off the plan; without its keys it
+// also publishes no count, so no other tile places its rows by one.  So none of them ranks the holes of this pass
 // against digit starts that were counted from all rows, and every position
 // written lies inside its digit's range.  (Reading plan->err at the start of
 // each tile instead cost 1.6% of a sort.)
@@ -600,7 +602,7 @@ __global__ void __launch_bounds__(OS_NT, 2) k_radix_onesweep(digit_of<KW, FLT> d
     if (!(full && kbulk)) {
         for (int i = t; i < tile_n; i += OS_NT) st_key<KW>(skeys, i, ld_key<KW>(kin, tile_base + i));
         __syncthreads();
-    } else if (!dev_::mbar_wait_bounded(bar0, 0, OS_COPY_WAIT)) {
+    } else if (!dev_::mbar_wait_bounded(bar0, 0, a.copy_limit)) {
         failed = 1;
     }
     if constexpr (VW > 0) {
@@ -624,7 +626,18 @@ __global__ void __launch_bounds__(OS_NT, 2) k_radix_onesweep(digit_of<KW, FLT> d
             rk[k] = warp_rank(wm, wh, d, valid, lane) | d << 16;
         }
     }
-    __syncthreads();
+    auto give_up = [&] {  // thread 0
+        atomicExch(&a.plan->err, 1);
+        for (int p = a.pass + 1; p < OS_MAX_PASSES; ++p) a.plan->order[p] = -1;
+        // Leave no copy in flight into this CTA's shared memory.
+        if (full && kbulk) dev_::mbar_wait_bounded(bar0, 0, OS_COPY_WAIT);
+        if (full && load_vals && vbulk) dev_::mbar_wait_bounded(bar1, 0, OS_COPY_WAIT);
+    };
+    if (__syncthreads_or(failed)) {  // the keys did not arrive
+        if (t < RS_BINS) st_state(state + tile * RS_BINS + t, OS_FAIL);
+        if (t == 0) give_up();
+        return;
+    }
 
     // Tile counts per digit; their prefix over the warps and over the digits.
     unsigned tot = 0, incl = 0;
@@ -691,15 +704,9 @@ __global__ void __launch_bounds__(OS_NT, 2) k_radix_onesweep(digit_of<KW, FLT> d
         if (tile > 0) st_state(state + tile * RS_BINS + t, failed ? OS_FAIL : OS_INC | (before + tot));
         gbase[t] = (int64_t)(a.plan->base[a.pass][t] + before) - (int64_t)ex;
     }
-    if (load_vals && full && vbulk && !dev_::mbar_wait_bounded(bar1, 0, OS_COPY_WAIT)) failed = 1;
+    if (load_vals && full && vbulk && !dev_::mbar_wait_bounded(bar1, 0, a.copy_limit)) failed = 1;
     if (__syncthreads_or(failed)) {
-        if (t == 0) {
-            atomicExch(&a.plan->err, 1);
-            for (int p = a.pass + 1; p < OS_MAX_PASSES; ++p) a.plan->order[p] = -1;
-            // Leave no copy in flight into this CTA's shared memory.
-            if (full && kbulk) dev_::mbar_wait_bounded(bar0, 0, OS_COPY_WAIT);
-            if (full && load_vals && vbulk) dev_::mbar_wait_bounded(bar1, 0, OS_COPY_WAIT);
-        }
+        if (t == 0) give_up();
         return;
     }
 #pragma unroll
@@ -868,7 +875,7 @@ int poll_limit(const char* name, int limit) {
     return e ? std::min(std::max(atoi(e), 0), limit) : limit;
 }
 
-// n > 0, begin_bit < end_bit.  Returns false when a look-back wait gave up
+// n > 0, begin_bit < end_bit.  Returns false when a wait gave up
 // (the outputs are then unspecified, the inputs untouched).
 template <int KW, int VW, bool FLT>
 bool onesweep_run(const col& keys, const void* vin, bool iota, const img_params& ip, int begin_bit, int end_bit,
@@ -915,6 +922,7 @@ bool onesweep_run(const col& keys, const void* vin, bool iota, const img_params&
     a.n = n;
     a.iota = iota ? 1 : 0;
     a.spin_limit = poll_limit("GX_RADIX_LOOKBACK_POLLS", OS_SPIN_LIMIT);
+    a.copy_limit = (uint32_t)poll_limit("GX_RADIX_COPY_POLLS", (int)OS_COPY_WAIT);
     a.plan = reinterpret_cast<os_plan*>(tp);
     tp += r256(sizeof(os_plan));
     a.state[0] = reinterpret_cast<os_state*>(tp);

@@ -107,10 +107,14 @@ def test_sort_one_cta_and_onesweep_edges(n, kdt, vdt):
 @pytest.mark.parametrize("n", [50_000, 512 * 4 * 300 + 7, 4608 * 148 * 5 + 1])
 @pytest.mark.parametrize("kdt,vdt", [(np.int32, np.int64), (np.float64, np.int32), (np.int64, np.int64)])
 @pytest.mark.parametrize("off", [0, 1])
-def test_sort_whose_look_back_gives_up(monkeypatch, n, kdt, vdt, off):
-    # Every tile but the first gives up at once (limit 0), or where the tile
-    # before it is late (limit 1): the passes that follow move nothing and the
-    # per-tile passes sort the untouched inputs.
+@pytest.mark.parametrize("wait", ["LOOKBACK", "COPY"])
+def test_sort_whose_waits_give_up(monkeypatch, n, kdt, vdt, off, wait):
+    # Every tile but the first gives up its look-back at once (limit 0), or
+    # where the tile before it is late (limit 1); or no full tile waits for the
+    # copy of its rows (columns off 16-byte boundaries are not copied).  The
+    # passes that follow move nothing and the per-tile passes sort the
+    # untouched inputs.
+    name = f"GX_RADIX_{wait}_POLLS"
     rng = np.random.default_rng(n)
     key = rng.integers(0, 256, size=(n + 1) * np.dtype(kdt).itemsize, dtype=np.uint8).view(kdt)
     if np.dtype(kdt).kind == "f":
@@ -132,12 +136,13 @@ def test_sort_whose_look_back_gives_up(monkeypatch, n, kdt, vdt, off):
         return used
 
     plain = launches_of_a_sort()
-    monkeypatch.setenv("GX_RADIX_LOOKBACK_POLLS", "0")
-    assert launches_of_a_sort() > plain  # the one-sweep passes and the per-tile ones
-    monkeypatch.setenv("GX_RADIX_LOOKBACK_POLLS", "1")
+    monkeypatch.setenv(name, "0")
+    if wait == "LOOKBACK" or off == 0:
+        assert launches_of_a_sort() > plain  # the one-sweep passes and the per-tile ones
+    monkeypatch.setenv(name, "1")
     launches_of_a_sort()
     assert np.array_equal(dk.cpu().numpy().view(np.uint8), key.view(np.uint8))
-    monkeypatch.delenv("GX_RADIX_LOOKBACK_POLLS")
+    monkeypatch.delenv(name)
     assert launches_of_a_sort() == plain
 
 
