@@ -9,6 +9,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cstdlib>
 #include <cstring>
 #include <memory>
 #include <stdexcept>
@@ -344,6 +345,12 @@ inline int ilog2_ceil(uint64_t x) {
     return b;
 }
 inline uint64_t next_pow2(uint64_t x) { return x <= 1 ? 1 : (uint64_t(1) << ilog2_ceil(x)); }
+// Polls before a device wait gives up: `limit`, or fewer where a test sets the
+// environment variable to make the wait run out.
+inline int poll_limit(const char* name, int limit) {
+    const char* e = getenv(name);
+    return e ? std::min(std::max(atoi(e), 0), limit) : limit;
+}
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 // Host <- device copy of at most HOST_READ_MAX bytes through the calling

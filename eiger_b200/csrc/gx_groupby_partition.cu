@@ -277,7 +277,8 @@ __global__ void __launch_bounds__(PS_NT, 2) k_part_scatter_r(const void* __restr
 // does; a tile that spans several values ranks them one after the other, a
 // barrier apart.  (Ranking every row in input order by __match_any_sync took
 // 1.8 ms per 2^28 rows alone, and its per-warp counts left no room for three
-// 8-byte columns.)  Each output
+// 8-byte columns.)  A first pass that gave up left holes, which are in no
+// order: the second pass then does nothing.  Each output
 // position j then reads its source row from the shared copy and writes every
 // column to gbase[digit] + j.  Used when every loaded column starts on a
 // 16-byte boundary and two tiles of the columns fit in shared memory.
@@ -313,7 +314,8 @@ template <int KW, int NC, bool SECOND>
 __global__ void __launch_bounds__(PB_NT, 1) k_part_scatter_bulk(const void* __restrict__ keys, int64_t n, int kind,
                                                                 int shift, int dbits, int64_t ntiles,
                                                                 const int64_t* __restrict__ offsets, move_cols mc,
-                                                                pb_layout L, int* __restrict__ err) {
+                                                                pb_layout L, uint32_t wait_limit,
+                                                                int* __restrict__ err) {
     extern __shared__ __align__(128) unsigned char pb_smem[];
     __shared__ __align__(8) unsigned long long bars[2];
     __shared__ unsigned wsum[PS_BINS / 32];
@@ -354,10 +356,11 @@ __global__ void __launch_bounds__(PB_NT, 1) k_part_scatter_bulk(const void* __re
         dev_::mbar_init(bar0, 1);
         dev_::mbar_init(bar0 + 8, 1);
         dev_::mbar_init_fence();
-        s_err = 0;
+        s_err = SECOND ? *(volatile int*)err : 0;
     }
     if (t < PS_BINS) thist[t] = 0;
     __syncthreads();
+    if (SECOND && s_err) return;
     // A copy into stage b was issued and not yet waited for: tracked by
     // thread 0, the only issuer.
     // Bit b of `pending` / `phase`: stage b's copy state and barrier parity.
@@ -377,7 +380,7 @@ __global__ void __launch_bounds__(PB_NT, 1) k_part_scatter_bulk(const void* __re
         // Digit offsets of this tile (read early; used after the scan).
         const int64_t my_off = t < bins ? offsets[(int64_t)t * ntiles + tile] : 0;
         if (full(tile)) {
-            if (dev_::mbar_wait_bounded(bar0 + 8u * (uint32_t)b, (phase >> b) & 1u, PB_WAIT_LIMIT)) {
+            if (dev_::mbar_wait_bounded(bar0 + 8u * (uint32_t)b, (phase >> b) & 1u, wait_limit)) {
                 phase ^= 1u << b;
                 pending &= ~(1u << b);
             } else {
@@ -817,10 +820,11 @@ void part_pass(const void* kin, int64_t n, int kind, int shift, int dbits, move_
             GX_CUDA(cudaFuncSetAttribute(k_part_scatter_bulk<KW, 4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
         });
         const int grid = (int)std::min<int64_t>(ntiles, dev().sm_count);
+        const uint32_t wait_limit = (uint32_t)poll_limit("GX_PART_COPY_POLLS", (int)PB_WAIT_LIMIT);
         GX_PROF("partition_scatter", s);
 #define GX_PB_LAUNCH(NCV, ST)                                                                                       \
     k_part_scatter_bulk<KW, NCV, ST><<<grid, PB_NT, L.total, s>>>(kin, n, kind, shift, dbits, ntiles, \
-                                                                          offs, mc, L, err)
+                                                                          offs, mc, L, wait_limit, err)
         if (mc.n == 2 && second) GX_PB_LAUNCH(2, true);
         else if (mc.n == 2) GX_PB_LAUNCH(2, false);
         else if (mc.n == 3 && second) GX_PB_LAUNCH(3, true);

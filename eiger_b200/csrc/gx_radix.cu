@@ -23,7 +23,6 @@
 // state: it serves the allocation-free sort, and a sort whose look-back gave
 // up runs through it again.
 #include <algorithm>
-#include <cstdlib>
 
 #include "gx_groupby.h"
 
@@ -867,12 +866,6 @@ size_t onesweep_temp_bytes(int64_t n, int kw, int vw) {
     return r256((size_t)n * kw) + r256((size_t)n * vw) + r256(sizeof(os_plan)) +
            2 * (size_t)ceil_div(n, (int64_t)OS_NT * (n >= (int64_t)1 << 19 ? OS_IPT_MIN : OS_IPT_SMALL)) * RS_BINS *
                sizeof(os_state);
-}
-
-// A wait's limit, or the shorter one that a test sets to make it run out.
-int poll_limit(const char* name, int limit) {
-    const char* e = getenv(name);
-    return e ? std::min(std::max(atoi(e), 0), limit) : limit;
 }
 
 // n > 0, begin_bit < end_bit.  Returns false when a wait gave up

@@ -161,6 +161,24 @@ def test_unique_sparse_keys_one_pass(algo, kdt, nb, npr):
                     assert np.array_equal(key[o], pk[er[e]])
 
 
+@pytest.mark.parametrize("kdt", [np.int32, np.int64])
+@pytest.mark.parametrize("nb", [1 << 17, 1 << 19])
+def test_partition_join_whose_copies_give_up(monkeypatch, kdt, nb):
+    # No wait for the copies of full tiles: the first pass (7 bits) or the first
+    # of two (9 bits) moves nothing and the join reports it; the next is whole.
+    bk = O.gen_perm(nb, kdt, seed=5) * kdt(3)
+    pk = O.gen_keys(2 * nb, kdt, groups=nb, seed=6, miss_frac=0.2) * kdt(3)
+    monkeypatch.setenv("GX_PART_COPY_POLLS", "0")
+    with pytest.raises(gx.GxError, match="did not complete"):
+        rowid_pairs(bk, pk, gx.JOIN_PARTITION)
+    monkeypatch.delenv("GX_PART_COPY_POLLS")
+    l, r = rowid_pairs(bk, pk, gx.JOIN_PARTITION)
+    m = O.join_probe_unique(bk, pk)
+    o = np.argsort(r, kind="stable")
+    hit = np.nonzero(m >= 0)[0]
+    assert np.array_equal(r[o], hit) and np.array_equal(l[o], m[hit])
+
+
 @pytest.mark.parametrize("algo", [gx.JOIN_SORT, gx.JOIN_HASH])
 @pytest.mark.parametrize("form", ["rowids", "table"])
 @pytest.mark.parametrize("npr,share", [(1 << 20, 0.05), (1 << 24, 0.05), (1 << 24, 0.45)])
