@@ -586,14 +586,17 @@ __global__ void k_starts_from_offsets(const int64_t* __restrict__ offs, int64_t 
     else if (p == P) ps[P] = n;
 }
 
-// Work units: partition p split into ceil(size/T) units.
+// Work units: partition p split into ceil(size/T) units.  None when the scatter
+// gave up (flags[0]): the rows are then in no order and some were not written,
+// so the partitions' starts need not ascend and row ids may be anything.
+// flags[1] counts the split partitions.
 __global__ void k_unit_counts(const int64_t* __restrict__ part_start, int P, int64_t T,
-                              int64_t* __restrict__ ucount, int* __restrict__ n_split) {
+                              int64_t* __restrict__ ucount, int* __restrict__ flags) {
     int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p < P) {
-        int64_t sz = part_start[p + 1] - part_start[p];
+        int64_t sz = flags[0] ? 0 : part_start[p + 1] - part_start[p];
         ucount[p] = sz == 0 ? 0 : (sz + T - 1) / T;
-        if (sz > T) atomicAdd(n_split, 1);
+        if (sz > T) atomicAdd(flags + 1, 1);
     }
 }
 using unit = part_unit;
@@ -962,8 +965,7 @@ void partition_groupby(const col& key_in, const agg_plan& p, gx_groupby_hint* hi
     // that about four units per SM exist.
     int64_t T = std::max<int64_t>(1 << 14, std::min<int64_t>(2 * ceil_div(n, P), ceil_div(n, (int64_t)dev().sm_count * 8)));
     dbuf ucount((size_t)P * 8, s);
-    k_unit_counts<<<(unsigned)ceil_div(P, 256), 256, 0, s>>>(pstart.get<int64_t>(), P, T, ucount.get<int64_t>(),
-                                                             perr + 1);
+    k_unit_counts<<<(unsigned)ceil_div(P, 256), 256, 0, s>>>(pstart.get<int64_t>(), P, T, ucount.get<int64_t>(), perr);
     GX_LAUNCHED();
     exclusive_scan_i64(ucount.get<int64_t>(), uoff.get<int64_t>(), P, s);
     int64_t max_units = P + ceil_div(n, T) + 1;

@@ -483,3 +483,28 @@ def test_runs_of_keys_seen_once_before(algo, kdt, G, run):
     # Sums in another order: at most n roundings of the sum of magnitudes.
     bound = n * 2.0**-53 * float(np.abs(fv).sum() / fv.sum())
     assert_columns_match(sort_by_key(t.numpy_columns()), list(exp), float_cols_rtol=max(1e-12, bound))
+
+
+@pytest.mark.parametrize("algo", [gx.PARTITION, gx.PARTITION_GFUR])
+@pytest.mark.parametrize("kdt", [np.int32, np.int64])
+@pytest.mark.parametrize("bits", [6, 12])
+@pytest.mark.parametrize("G", [5_000, 400_000])
+def test_partition_whose_copies_give_up(monkeypatch, algo, kdt, bits, G):
+    # No wait for the copies of full tiles, in one pass and the first of two:
+    # nothing is aggregated and the call reports it (with a small table for all
+    # groups at its end, with a large one before); the next call is whole.
+    n = 4096 * 200 + 99
+    key = O.gen_keys(n, kdt, groups=G, seed=71) * kdt(3)
+    iv, fv = O.gen_values(n, np.int64, lo=0, hi=1000, seed=72), O.gen_values(n, np.float64, seed=73)
+    ops = [(0, "SUM"), (1, "MAX"), (0, "COUNT_ALL")]
+
+    def run():
+        return gx.groupby([to_dev(key)], [to_dev(iv), to_dev(fv)], [(c, getattr(gx, o)) for c, o in ops],
+                          gx.make_hint(algo, G, radix_bits=bits))
+
+    monkeypatch.setenv("GX_PART_COPY_POLLS", "0")
+    with pytest.raises(gx.GxError, match="did not complete"):
+        run()
+    monkeypatch.delenv("GX_PART_COPY_POLLS")
+    assert_columns_match(sort_by_key(run().numpy_columns()),
+                         list(O.groupby(key, [iv, fv], [(c, getattr(O, o)) for c, o in ops])))
