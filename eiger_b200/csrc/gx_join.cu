@@ -387,6 +387,14 @@ __device__ __forceinline__ int64_t lookback(unsigned long long* tstate, int64_t 
     return excl;
 }
 
+// Tile of a CTA that probes unique build keys, -1 where the build kernel found
+// duplicates (its flag lies behind the look-back's) and the probe is void.
+__device__ __forceinline__ int64_t take_tile(unsigned* ticket, const int* err) {
+    const int dup = *(volatile const int*)(err + 1);
+    const unsigned tile = atomicAdd(ticket, 1u);
+    return dup ? -1 : (int64_t)tile;
+}
+
 // ROWIDS: the output is just the (build row, probe row) pair (int64 each).
 template <int KW, bool ROWIDS>
 __global__ void __launch_bounds__(JP_NT) k_dense_probe1(const void* __restrict__ pkeys, int64_t np, int kind,
@@ -399,9 +407,10 @@ __global__ void __launch_bounds__(JP_NT) k_dense_probe1(const void* __restrict__
     __shared__ int64_t sm[JP_NT / 32 + 1];
     __shared__ int64_t s_tile, s_excl;
     __shared__ int s_skip;
-    if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
+    if (threadIdx.x == 0) s_tile = take_tile(ticket, err);
     __syncthreads();
     const int64_t tile = s_tile;
+    if (tile < 0) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int64_t row0 = tile * (int64_t)JP_TILE + warp * 32 * JP_IPT + lane;
     uint32_t m[JP_IPT];
@@ -603,9 +612,10 @@ __global__ void __launch_bounds__(UH_NT, SW == 8 ? 4 : 3) k_uniq_probe(const uns
     __shared__ int64_t sm[UH_NT / 32 + 1];
     __shared__ int64_t s_tile, s_excl;
     __shared__ int s_skip;
-    if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
+    if (threadIdx.x == 0) s_tile = take_tile(ticket, err);
     __syncthreads();
     const int64_t tile = s_tile;
+    if (tile < 0) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t row0 = tile * (int64_t)UH_TILE + warp * 32 * UH_IPT + lane;
     kt key[UH_IPT];
@@ -947,11 +957,13 @@ static void join_core(const join_inputs& in, const gx_join_hint& hint, bool rowi
     if (nb > 0) key_image_range(bkey, &lo, &hi, s);
     uint64_t span = hi - lo;
     // Dense unique build keys: place rows by key instead of comparison sorting.
-    if (nb > 0 && hint.sort_mode == GX_JOIN_SORTED_BUILD && nb < (int64_t)NO_ROW && span < (uint64_t)nb * 4 &&
-        dense_join(in, hint, rowids_only, build_left, lo, hi, s, out))
-        return;
+    bool may_be_unique = true;
+    if (nb > 0 && hint.sort_mode == GX_JOIN_SORTED_BUILD && nb < (int64_t)NO_ROW && span < (uint64_t)nb * 4) {
+        if (dense_join(in, hint, rowids_only, build_left, lo, hi, s, out)) return;
+        may_be_unique = false;
+    }
     static const bool two_pass = getenv("GX_JOIN_TWO_PASS") != nullptr;
-    if (hint.sort_mode == GX_JOIN_SORTED_BUILD && !two_pass &&
+    if (hint.sort_mode == GX_JOIN_SORTED_BUILD && !two_pass && may_be_unique &&
         unique_hash_join(in, hint, rowids_only, build_left, s, out))
         return;
     // Sort the build side: (key, payload) when exactly one 4/8-byte payload.
