@@ -59,42 +59,50 @@ __device__ __forceinline__ T bound_of(uint64_t bits) {
     else return (T)bits;
 }
 
-// Bit k: row row0 + 32 k (below n) is in the range of predicate j.  float32
-// values are compared as doubles: the literal need not be a float.
+// Bit k: row row0 + 32 k is in the range of predicate j, for the rows of `need`
+// (no other is read).  float32 values are compared as doubles: the literal
+// need not be a float.
 template <class T>
-__device__ __forceinline__ unsigned range_bits(const pred_dev& p, int j, int64_t row0, int64_t n) {
+__device__ __forceinline__ unsigned range_bits(const pred_dev& p, int j, int64_t row0, unsigned need) {
     using C = typename std::conditional<std::is_same<T, float>::value, double, T>::type;
     const T* d = static_cast<const T*>(p.data[j]);
     const C lo = bound_of<C>(p.lo[j]), hi = bound_of<C>(p.hi[j]);
     T x[SL_IPT];
 #pragma unroll
-    for (int k = 0; k < SL_IPT; ++k) x[k] = row0 + k * 32 < n ? __ldg(d + row0 + k * 32) : T(0);
+    for (int k = 0; k < SL_IPT; ++k) x[k] = (need >> k) & 1u ? __ldg(d + row0 + k * 32) : T(0);
     unsigned b = 0;
 #pragma unroll
     for (int k = 0; k < SL_IPT; ++k) b |= ((C)x[k] >= lo && (C)x[k] <= hi ? 1u : 0u) << k;
     return p.negate[j] ? ~b : b;
 }
 
+// Whole warps.  A predicate after the first reads only rows that it decides
+// (AND: kept so far, OR: not yet), and none when a warp has no such row.  2^26
+// rows, eight 8-byte columns under AND, the first predicate true for 1 in 10^5
+// rows: 200 us a call, 710 when every predicate read every row.
 __device__ __forceinline__ unsigned keep_bits(const pred_dev& p, int64_t row0, int64_t n) {
-    unsigned keep = p.combine == 0 ? ~0u : 0u;
+    const int64_t rows = (n - row0 + 31) >> 5;  // of this thread, below n
+    const unsigned valid = rows >= SL_IPT ? (1u << SL_IPT) - 1u : rows <= 0 ? 0u : (1u << rows) - 1u;
+    unsigned keep = p.combine == 0 ? valid : 0u;
     for (int j = 0; j < p.n; ++j) {
+        const unsigned need = p.combine == 0 ? keep : valid & ~keep;
+        if (!__any_sync(0xffffffffu, need)) break;
         unsigned b;
         switch (p.type[j]) {
-            case GX_INT8: b = range_bits<signed char>(p, j, row0, n); break;
-            case GX_INT16: b = range_bits<short>(p, j, row0, n); break;
-            case GX_INT32: b = range_bits<int>(p, j, row0, n); break;
-            case GX_INT64: b = range_bits<long long>(p, j, row0, n); break;
-            case GX_UINT16: b = range_bits<unsigned short>(p, j, row0, n); break;
-            case GX_UINT32: b = range_bits<unsigned>(p, j, row0, n); break;
-            case GX_UINT64: b = range_bits<unsigned long long>(p, j, row0, n); break;
-            case GX_FLOAT32: b = range_bits<float>(p, j, row0, n); break;
-            case GX_FLOAT64: b = range_bits<double>(p, j, row0, n); break;
-            default: b = range_bits<unsigned char>(p, j, row0, n); break;  // UINT8, BOOL8
+            case GX_INT8: b = range_bits<signed char>(p, j, row0, need); break;
+            case GX_INT16: b = range_bits<short>(p, j, row0, need); break;
+            case GX_INT32: b = range_bits<int>(p, j, row0, need); break;
+            case GX_INT64: b = range_bits<long long>(p, j, row0, need); break;
+            case GX_UINT16: b = range_bits<unsigned short>(p, j, row0, need); break;
+            case GX_UINT32: b = range_bits<unsigned>(p, j, row0, need); break;
+            case GX_UINT64: b = range_bits<unsigned long long>(p, j, row0, need); break;
+            case GX_FLOAT32: b = range_bits<float>(p, j, row0, need); break;
+            case GX_FLOAT64: b = range_bits<double>(p, j, row0, need); break;
+            default: b = range_bits<unsigned char>(p, j, row0, need); break;  // UINT8, BOOL8
         }
-        keep = p.combine == 0 ? keep & b : keep | b;
+        keep = p.combine == 0 ? keep & b : keep | (need & b);
     }
-    const int64_t rows = (n - row0 + 31) >> 5;  // of this thread, below n
-    return keep & (rows >= SL_IPT ? (1u << SL_IPT) - 1u : rows <= 0 ? 0u : (1u << rows) - 1u);
+    return keep;
 }
 
 // Row (k, lane) of warp w in tile t: t*TILE + w*32*IPT + k*32 + lane.

@@ -111,3 +111,25 @@ def test_float_ranges_with_infinities_nan_and_zeros(dt):
                 assert np.array_equal(gx.select_to_bitmask([d], [p]).cpu().numpy().astype(bool), e), (op, lo, hi)
                 got = gx.select([d], [p]).to_numpy(0)
                 assert np.array_equal(got, a[e], equal_nan=True), (op, lo, hi)
+
+
+@pytest.mark.parametrize("combine", [gx.COMBINE_AND, gx.COMBINE_OR])
+@pytest.mark.parametrize("n", [1, 33, 511, 512, 513, 4097, 100_003])
+@pytest.mark.parametrize("decided", [0.0, 0.9, 0.9999, 1.0])
+def test_rows_decided_by_the_first_predicate(combine, n, decided):
+    # Rows that the first predicate decides (false under AND, true under OR) are
+    # not read by the later ones, whole warps of them or single rows.
+    rng = np.random.default_rng(n)
+    a = (rng.random(n) < decided).astype(np.int8)
+    a[n // 2:] = a[n // 2:] if decided < 0.99 else 1  # long decided stretches
+    b = rng.integers(0, 10, n).astype(np.uint16)
+    c = np.where(rng.random(n) < 0.2, np.nan, rng.random(n)).astype(np.float32)
+    cols = [to_dev(a), to_dev_raw(b), to_dev(c)]
+    views = [gx.ColumnView(t.data_ptr(), n, gx._NP_TO_GX[x.dtype], 0) for t, x in zip(cols, (a, b, c))]
+    first = gx.predicate(0, gx.CMP_EQ, 0 if combine == gx.COMBINE_AND else 1)
+    preds = [first, gx.predicate(1, gx.CMP_NE, 4), gx.predicate(2, gx.CMP_LT, 0.5)]
+    parts = [a == (0 if combine == gx.COMBINE_AND else 1), b != 4, c < 0.5]
+    keep = np.logical_and.reduce(parts) if combine == gx.COMBINE_AND else np.logical_or.reduce(parts)
+    assert np.array_equal(gx.select_to_bitmask(views, preds, combine).cpu().numpy().astype(bool), keep)
+    for got, x in zip(gx.select(views, preds, combine).numpy_columns(), (a, b, c)):
+        assert np.array_equal(got, x[keep], equal_nan=x.dtype.kind == "f")
