@@ -543,59 +543,49 @@ __global__ void __launch_bounds__(JP_NT) k_sorted_probe1(build_run b, probe_side
 // slots at load 1/4 to 1/2, probed in one pass.  A probe row then costs one or
 // two random sectors (its slot holds the key and what the output needs of the
 // build row) where the sorted run costs a directory entry, a bucket's keys and
-// a value, and the build side is not sorted.  Slots: 8 bytes (key << 32 | row)
-// for 4-byte keys whose output needs the build row; else 16 bytes (key, the
-// one payload or the row).  Rows come out in probe order, as from the sorted
-// run.  10^6 sparse int64 keys and payloads joined to 3 * 10^7 rows with
+// a value, and the build side is not sorted.  Slots: see key_table.  Rows come
+// out in probe order, as from the sorted run.  10^6 sparse int64 keys and payloads joined to 3 * 10^7 rows with
 // payloads: 0.99 ms a call, 1.55 ms through the sorted run.
-// Duplicated build keys, and an 8-byte key equal to the empty marker, set
-// *bad; the caller then takes its other plan.
+// Duplicated build keys (UH_DUP), and an 8-byte key equal to the empty marker
+// (UH_MARKER), set *bad; the caller then takes its other plan.  Unless
+// `multi`, where duplicates take a slot each, the build ends there.
 // ---------------------------------------------------------------------------
-constexpr unsigned long long UH_EMPTY8 = ~0ull;                  // 8-byte slot: row 2^32 - 1
-constexpr unsigned long long UH_EMPTY4K = ~0ull;                 // 16-byte slot, 4-byte keys (zero-extended)
-constexpr unsigned long long UH_EMPTY8K = 0x8000000000000000ull; // 16-byte slot, 8-byte keys
+constexpr int UH_DUP = 1, UH_MARKER = 2;
 constexpr int UH_NT = 256;
 constexpr int UH_IPT = 8;
 constexpr int UH_TILE = UH_NT * UH_IPT;
-
-template <int KW>
-__device__ __forceinline__ uint64_t uh_hash(uint64_t k) {
-    if (KW == 4) return fmix32((uint32_t)k);
-    return fmix64(k);
-}
-template <int KW>
-__device__ __forceinline__ unsigned long long uh_empty() {
-    return KW == 4 ? UH_EMPTY4K : UH_EMPTY8K;
-}
 
 // pay: the build payload column (width 4 or 8) or null (value = row).
 template <int KW, int SW>
 __global__ void __launch_bounds__(UH_NT) k_uniq_build(const void* __restrict__ keys, const void* __restrict__ pay,
                                                       int pay_width, int64_t n, unsigned long long* __restrict__ table,
-                                                      uint64_t mask, int* __restrict__ bad) {
+                                                      uint64_t mask, int multi, int* __restrict__ bad) {
+    constexpr unsigned long long EMPTY = uh_empty<KW, SW>();
+    bool dup = false;
     for (int64_t i = blockIdx.x * (int64_t)UH_NT + threadIdx.x; i < n; i += (int64_t)gridDim.x * UH_NT) {
-        if (*(volatile int*)bad) return;
+        if (*(volatile int*)bad > (multi ? UH_DUP : 0)) return;
         unsigned long long k;
         if (KW == 4) k = __ldg(static_cast<const unsigned*>(keys) + i);
         else k = __ldg(static_cast<const unsigned long long*>(keys) + i);
-        if (KW == 8 && k == UH_EMPTY8K) { atomicExch(bad, 1); return; }
+        if (KW == 8 && k == UH_EMPTY8K) { atomicOr(bad, UH_MARKER); return; }
         uint64_t slot = uh_hash<KW>(k) & mask & ~uint64_t(1);
         for (;;) {  // ends: the table is at most half full
-            if constexpr (SW == 8) {
-                const unsigned long long old = atomicCAS(table + slot, UH_EMPTY8, k << 32 | (unsigned)i);
-                if (old == UH_EMPTY8) break;
-                if (old >> 32 == k) { atomicExch(bad, 1); return; }
-            } else {
-                const unsigned long long old = atomicCAS(table + 2 * slot, uh_empty<KW>(), k);
-                if (old == uh_empty<KW>()) {
+            unsigned long long old;
+            if constexpr (SW == 8) old = atomicCAS(table + slot, EMPTY, k << 32 | (unsigned)i);
+            else old = atomicCAS(table + 2 * slot, EMPTY, k);
+            if (old == EMPTY) {
+                if constexpr (SW == 16)
                     table[2 * slot + 1] = !pay ? (unsigned long long)i : (unsigned long long)ld_w(pay, pay_width, i);
-                    break;
-                }
-                if (old == k) { atomicExch(bad, 1); return; }
+                break;
+            }
+            if ((SW == 8 ? old >> 32 : old) == k) {
+                if (!multi) { atomicOr(bad, UH_DUP); return; }
+                dup = true;
             }
             slot = (slot + 1) & mask;
         }
     }
+    if (dup) atomicOr(bad, UH_DUP);
 }
 
 // Sources: 0 and 3 = the slot's value, 1 = build column at the build row (the
@@ -634,7 +624,7 @@ __global__ void __launch_bounds__(UH_NT, SW == 8 ? 4 : 3) k_uniq_probe(const uns
     // unresolved row at once; the table is at most half full, so every walk
     // meets an empty slot.  The second slot of a pair is only filled after the
     // first, so an empty first slot ends a walk too.
-    constexpr unsigned long long EMPTY = SW == 8 ? UH_EMPTY8 : KW == 4 ? UH_EMPTY4K : UH_EMPTY8K;
+    constexpr unsigned long long EMPTY = uh_empty<KW, SW>();
     while (open) {
         unsigned long long w0[UH_IPT], w1[UH_IPT];
 #pragma unroll
@@ -873,7 +863,7 @@ static void shrink_outputs(gx_table* out, int64_t cap, int64_t total, cudaStream
 }
 
 bool unique_hash_join(const join_inputs& in, const gx_join_hint& hint, bool rowids_only, bool build_left,
-                      cudaStream_t s, gx_table* out) {
+                      cudaStream_t s, gx_table* out, key_table* dup) {
     const col& bkey = build_left ? in.lkey : in.rkey;
     const col& pkey = build_left ? in.rkey : in.lkey;
     const std::vector<col>& bpay = build_left ? in.lpay : in.rpay;
@@ -885,6 +875,12 @@ bool unique_hash_join(const join_inputs& in, const gx_join_hint& hint, bool rowi
     const uint64_t cap = next_pow2(std::max<uint64_t>((uint64_t)nb * 2, 4));
     const int64_t ntiles = ceil_div(np, UH_TILE);
     const size_t table_bytes = (size_t)cap * sw;
+    // Duplicates are kept where the table fits in L2.  2^25 rows joined to keys
+    // twice each, ms a call, kept / in records by themselves: 2^20 int64 keys
+    // (32 MB) 5.37 / 5.88, 2^21 int32 (32 MB) 4.55 / 4.67, 2^22 int32 (64 MB)
+    // 4.96 / 4.92, 2^22 int64 (128 MB) 6.63 / 6.79, 2^23 int32 (128 MB) 5.93 /
+    // 5.76, 2^24 int64 (512 MB) 11.95 / 10.80.
+    const bool multi = dup && table_bytes <= (size_t)dev().l2_bytes;
     try {
         // Table, tile states, ticket, then total, error flag and build flag.
         dbuf table(table_bytes, s), ctl((size_t)ntiles * 8 + 32, s);
@@ -902,12 +898,24 @@ bool unique_hash_join(const join_inputs& in, const gx_join_hint& hint, bool rowi
         {
             GX_PROF("join_build_hash", s);
             const int g = grid_for(nb, UH_NT, 8);
-            if (sw == 8) k_uniq_build<4, 8><<<g, UH_NT, 0, s>>>(bkey.data, pay, pw, nb, tb, cap - 1, bad);
-            else if (kw == 4) k_uniq_build<4, 16><<<g, UH_NT, 0, s>>>(bkey.data, pay, pw, nb, tb, cap - 1, bad);
-            else k_uniq_build<8, 16><<<g, UH_NT, 0, s>>>(bkey.data, pay, pw, nb, tb, cap - 1, bad);
+            if (sw == 8) k_uniq_build<4, 8><<<g, UH_NT, 0, s>>>(bkey.data, pay, pw, nb, tb, cap - 1, multi, bad);
+            else if (kw == 4) k_uniq_build<4, 16><<<g, UH_NT, 0, s>>>(bkey.data, pay, pw, nb, tb, cap - 1, multi, bad);
+            else k_uniq_build<8, 16><<<g, UH_NT, 0, s>>>(bkey.data, pay, pw, nb, tb, cap - 1, multi, bad);
             GX_LAUNCHED();
         }
-        if (np > PROBE_AHEAD && read_scalar(bad, s)) return false;
+        auto not_unique = [&](int flags) {
+            out->cols.clear();
+            if (!multi || flags != UH_DUP) return false;
+            dup->slots = std::move(table);
+            dup->mask = cap - 1;
+            dup->width = sw;
+            dup->pay_in_run = pay_in_run;
+            return false;
+        };
+        if (np > PROBE_AHEAD) {
+            const int flags = read_scalar(bad, s);
+            if (flags) return not_unique(flags);
+        }
         join_out o = make_outputs(in, build_left, rowids_only, pay_in_run, false, np, s, out, np);
         {
             GX_PROF("join_probe_write", s);
@@ -919,7 +927,8 @@ bool unique_hash_join(const join_inputs& in, const gx_join_hint& hint, bool rowi
         }
         int64_t hs[2];
         host_read(hs, total_out, 16, s);
-        if (hs[1]) {  // a look-back wait gave up (low half), or the build flag (high half)
+        if (hs[1] >> 32) return not_unique((int)(hs[1] >> 32));
+        if (hs[1]) {  // a look-back wait gave up
             out->cols.clear();
             return false;
         }

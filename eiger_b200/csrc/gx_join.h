@@ -44,13 +44,38 @@ void hash_join(const join_inputs& in, const gx_join_hint& hint, bool rowids_only
 void partition_hash_join(const join_inputs& in, const gx_join_hint& hint, bool rowids_only, cudaStream_t s,
                          gx_table* out);
 
+// Hash table of integer build keys.  Slots: 8 bytes (key << 32 | row) for 4-byte
+// keys whose output needs the build row; else 16 bytes (key, value), the value
+// being the one payload (pay_in_run) or the row.  Rows with equal keys take a
+// slot each.  A key's walk starts at its hash with the lowest bit cleared and
+// ends at an empty slot: the table is at most half full.
+struct key_table {
+    dbuf slots;
+    uint64_t mask = 0;
+    int width = 0;  // bytes of a slot
+    bool pay_in_run = false;
+};
+
 // One-pass join of unique integer build keys through a hash table (gx_join.cu).
 // Returns false, with no output, when the build keys are not unique integers
-// or memory is short: the caller takes another plan.
+// or memory is short: the caller takes another plan.  With `dup`, a table whose
+// keys are not unique is completed and left there if it fits in L2.
 bool unique_hash_join(const join_inputs& in, const gx_join_hint& hint, bool rowids_only, bool build_left,
-                      cudaStream_t s, gx_table* out);
+                      cudaStream_t s, gx_table* out, key_table* dup = nullptr);
 
 #ifdef __CUDACC__
+constexpr unsigned long long UH_EMPTY8 = ~0ull;                  // 8-byte slot: row 2^32 - 1
+constexpr unsigned long long UH_EMPTY4K = ~0ull;                 // 16-byte slot, 4-byte keys (zero-extended)
+constexpr unsigned long long UH_EMPTY8K = 0x8000000000000000ull; // 16-byte slot, 8-byte keys
+template <int KW, int SW>
+__device__ __forceinline__ constexpr unsigned long long uh_empty() {
+    return SW == 8 ? UH_EMPTY8 : KW == 4 ? UH_EMPTY4K : UH_EMPTY8K;
+}
+template <int KW>
+__device__ __forceinline__ uint64_t uh_hash(uint64_t k) {
+    if (KW == 4) return fmix32((uint32_t)k);
+    return fmix64(k);
+}
 __device__ __forceinline__ uint64_t ld_w(const void* p, int w, int64_t i) {
     switch (w) {
         case 8: return __ldg(static_cast<const unsigned long long*>(p) + i);
@@ -69,7 +94,8 @@ __device__ __forceinline__ void st_w(void* p, int w, int64_t i, uint64_t v) {
     }
 }
 // One matched pair's output row: sources 1 = build column at the build row,
-// 2 = probe column at the probe row, 3 = build row id, 4 = probe row id; the
+// 2 = probe column at the probe row, 3 = build row id, 4 = probe row id; 0 =
+// `brow` itself, the payload where a table holds it in the row's place.  The
 // key column takes the probe row's key.
 __device__ __forceinline__ void write_pair(const join_out& o, const void* pkeys, int64_t pos, int64_t brow,
                                            int64_t prow) {
@@ -79,6 +105,7 @@ __device__ __forceinline__ void write_pair(const join_out& o, const void* pkeys,
         switch (o.src[c]) {
             case 1: v = ld_w(o.col[c], o.width[c], brow); break;
             case 2: v = ld_w(o.col[c], o.width[c], prow); break;
+            case 0:
             case 3: v = (uint64_t)brow; break;
             default: v = (uint64_t)prow; break;
         }

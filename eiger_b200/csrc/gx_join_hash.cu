@@ -14,14 +14,15 @@
 // order.
 //
 // B200 design:
-//   * HASH: unique integer build keys go through unique_hash_join (gx_join.cu,
-//     one probe pass); otherwise one open-addressing multiset of (key, build row) records at load
-//     <= 1/2, built with one 64-bit compare-and-swap per row (4-byte keys
-//     pack key and row in one record; 8-byte keys claim the row word and then
-//     store the key), probed in 2048-row tiles: a count kernel sizes every
-//     tile's output exactly, an exclusive scan places the tiles, and a write
-//     kernel emits the pairs.  Each thread issues its eight rows' home-slot
-//     loads together.  No atomics on the probe side, no output wrap.
+//   * HASH: integer build keys go into a key_table (gx_join.cu).  Unique ones
+//     are probed in one pass; a table with duplicates, and the multiset of
+//     (key, build row) records that other keys go into (load <= 1/2, one 64-bit
+//     compare-and-swap per row; 4-byte keys pack key and row in one record,
+//     8-byte keys claim the row word and then store the key), are probed in
+//     2048-row tiles: a count kernel sizes every tile's output exactly, an
+//     exclusive scan places the tiles, and a write kernel emits the pairs.
+//     Each thread issues its eight rows' home-slot loads together.  No atomics
+//     on the probe side, no output wrap.
 //   * PARTITION: both sides are radix-partitioned (key + row id) by the hash
 //     bits the PARTITION group-by uses, so that a build partition averages
 //     ~1024 rows; one CTA per partition loads the build rows into a
@@ -73,23 +74,50 @@ __global__ void k_hj_build(const void* __restrict__ bkeys, int64_t nb, int kind,
     }
 }
 
-// Walks the probe sequence of key k from `slot`; calls f(build_row) for
-// every equal key.  Returns the number of matches.
-template <int KW, class F>
-__device__ __forceinline__ int hj_walk(const unsigned long long* __restrict__ table, uint64_t mask, uint64_t slot,
-                                       uint64_t k, unsigned long long first, F&& f) {
+// The tables a probe walks.  `first` is the slot a walk starts at, `word` the
+// slot's first word, `hit` whether a full slot holds key k, `row` what the
+// output takes from it.
+template <int KW_>
+struct record_table {  // k_hj_build's records
+    static constexpr int KW = KW_;
+    static constexpr unsigned long long EMPTY = HJ_EMPTY;
+    const unsigned long long* t;
+    uint64_t mask;
+    __device__ __forceinline__ uint64_t first(uint64_t k) const { return hj_hash<KW>(k) & mask; }
+    __device__ __forceinline__ unsigned long long word(uint64_t s) const { return __ldg(t + (KW == 4 ? s : 2 * s)); }
+    __device__ __forceinline__ bool hit(unsigned long long w, uint64_t s, uint64_t k) const {
+        return KW == 4 ? (uint32_t)w == (uint32_t)k : __ldg(t + 2 * s + 1) == k;
+    }
+    __device__ __forceinline__ int64_t row(unsigned long long w, uint64_t) const {
+        return KW == 4 ? (int64_t)(w >> 32) : (int64_t)w;
+    }
+};
+template <int KW_, int SW>
+struct slot_table {  // a key_table
+    static constexpr int KW = KW_;
+    static constexpr unsigned long long EMPTY = uh_empty<KW, SW>();
+    const unsigned long long* t;
+    uint64_t mask;
+    __device__ __forceinline__ uint64_t first(uint64_t k) const { return uh_hash<KW>(k) & mask & ~uint64_t(1); }
+    __device__ __forceinline__ unsigned long long word(uint64_t s) const { return __ldg(t + (SW == 8 ? s : 2 * s)); }
+    __device__ __forceinline__ bool hit(unsigned long long w, uint64_t, uint64_t k) const {
+        return (SW == 8 ? w >> 32 : w) == k;
+    }
+    __device__ __forceinline__ int64_t row(unsigned long long w, uint64_t s) const {
+        return SW == 8 ? (int64_t)(uint32_t)w : (int64_t)__ldg(t + 2 * s + 1);
+    }
+};
+
+// Walks the probe sequence of key k from `slot`; calls f(row) for every equal
+// key.  Returns the number of matches.
+template <class T, class F>
+__device__ __forceinline__ int hj_walk(const T& t, uint64_t slot, uint64_t k, unsigned long long first, F&& f) {
     int c = 0;
-    unsigned long long rec = first;
-    for (;;) {
-        if (KW == 4) {
-            if (rec == HJ_EMPTY) break;
-            if ((uint32_t)rec == (uint32_t)k) { f((int64_t)(rec >> 32)); ++c; }
-        } else {
-            if (rec == HJ_EMPTY) break;
-            if (__ldg(table + 2 * slot + 1) == k) { f((int64_t)rec); ++c; }
-        }
-        slot = (slot + 1) & mask;
-        rec = __ldg(table + (KW == 4 ? slot : 2 * slot));
+    unsigned long long w = first;
+    while (w != T::EMPTY) {
+        if (t.hit(w, slot, k)) { f(w, slot); ++c; }
+        slot = (slot + 1) & t.mask;
+        w = t.word(slot);
     }
     return c;
 }
@@ -97,9 +125,8 @@ __device__ __forceinline__ int hj_walk(const unsigned long long* __restrict__ ta
 // Count (WRITE = false: per-tile match totals) or write (WRITE = true: pairs
 // at tile_off[tile] + the row-order prefix inside the tile).  Warp w of a
 // block owns rows [tile + w*32*IPT, +32*IPT); row (k, lane) = k*32 + lane.
-template <int KW, bool WRITE>
-__global__ void __launch_bounds__(HJ_NT) k_hj_probe(const unsigned long long* __restrict__ table, uint64_t mask,
-                                                     const void* __restrict__ pkeys, int64_t np, int kind,
+template <class T, bool WRITE>
+__global__ void __launch_bounds__(HJ_NT) k_hj_probe(T t, const void* __restrict__ pkeys, int64_t np, int kind,
                                                      int64_t* __restrict__ tile_cnt,
                                                      const int64_t* __restrict__ tile_off, join_out o) {
     __shared__ int64_t sm[HJ_NT / 32 + 1];
@@ -110,17 +137,16 @@ __global__ void __launch_bounds__(HJ_NT) k_hj_probe(const unsigned long long* __
 #pragma unroll
     for (int j = 0; j < HJ_IPT; ++j) {
         const int64_t i = row0 + j * 32;
-        k[j] = i < np ? hj_key<KW>(pkeys, i, kind) : 0;
-        slot[j] = hj_hash<KW>(k[j]) & mask;
+        k[j] = i < np ? hj_key<T::KW>(pkeys, i, kind) : 0;
+        slot[j] = t.first(k[j]);
     }
 #pragma unroll
-    for (int j = 0; j < HJ_IPT; ++j)
-        first[j] = row0 + j * 32 < np ? __ldg(table + (KW == 4 ? slot[j] : 2 * slot[j])) : HJ_EMPTY;
+    for (int j = 0; j < HJ_IPT; ++j) first[j] = row0 + j * 32 < np ? t.word(slot[j]) : T::EMPTY;
     int cnt[HJ_IPT];
     int64_t mine = 0;
 #pragma unroll
     for (int j = 0; j < HJ_IPT; ++j) {
-        cnt[j] = hj_walk<KW>(table, mask, slot[j], k[j], first[j], [](int64_t) {});
+        cnt[j] = hj_walk(t, slot[j], k[j], first[j], [](unsigned long long, uint64_t) {});
         mine += cnt[j];
     }
     const int64_t wtot = dev_::warp_sum(mine);
@@ -128,9 +154,9 @@ __global__ void __launch_bounds__(HJ_NT) k_hj_probe(const unsigned long long* __
         if (lane == 0) sm[warp] = wtot;
         __syncthreads();
         if (threadIdx.x == 0) {
-            int64_t t = 0;
-            for (int w = 0; w < HJ_NT / 32; ++w) t += sm[w];
-            tile_cnt[blockIdx.x] = t;
+            int64_t total = 0;
+            for (int w = 0; w < HJ_NT / 32; ++w) total += sm[w];
+            tile_cnt[blockIdx.x] = total;
         }
     } else {
         int64_t total;
@@ -144,8 +170,8 @@ __global__ void __launch_bounds__(HJ_NT) k_hj_probe(const unsigned long long* __
             running += __shfl_sync(0xffffffffu, inc, 31);
             const int64_t prow = row0 + j * 32;
             if (cnt[j])
-                hj_walk<KW>(table, mask, slot[j], k[j], first[j],
-                            [&](int64_t brow) { write_pair(o, pkeys, pos++, brow, prow); });
+                hj_walk(t, slot[j], k[j], first[j],
+                        [&](unsigned long long w, uint64_t at) { write_pair(o, pkeys, pos++, t.row(w, at), prow); });
         }
     }
 }
@@ -247,13 +273,49 @@ void check_max_out(const gx_join_hint& hint, int64_t total) {
 
 }  // namespace
 
+// Count, scan and write over a table of the build rows.
+template <class T>
+static void hj_join(const T& t, const join_inputs& in, const sides& sd, const gx_join_hint& hint, bool rowids_only,
+                    bool pay_in_run, cudaStream_t s, gx_table* out) {
+    const int64_t np = sd.pkey->n;
+    const int kind = vkind_of(in.lkey.type);
+    const int64_t ntiles = ceil_div(std::max<int64_t>(np, 1), HJ_TILE);
+    dbuf tc((size_t)ntiles * 8, s), toff((size_t)(ntiles + 1) * 8, s);
+    int64_t total = 0;
+    join_out none;
+    std::memset(&none, 0, sizeof(none));
+    if (np > 0 && sd.bkey->n > 0) {
+        GX_PROF("join_probe_count", s);
+        k_hj_probe<T, false><<<(unsigned)ntiles, HJ_NT, 0, s>>>(t, sd.pkey->data, np, kind, tc.get<int64_t>(), nullptr, none);
+        GX_LAUNCHED();
+        exclusive_scan_i64(tc.get<int64_t>(), toff.get<int64_t>(), ntiles, s);
+        total = read_scalar(toff.get<int64_t>() + ntiles, s);
+    }
+    check_max_out(hint, total);
+    join_out o = make_outputs(in, sd.build_left, rowids_only, pay_in_run, !pay_in_run, total, s, out);
+    if (total > 0) {
+        GX_PROF("join_probe_write", s);
+        k_hj_probe<T, true><<<(unsigned)ntiles, HJ_NT, 0, s>>>(t, sd.pkey->data, np, kind, nullptr, toff.get<int64_t>(), o);
+        GX_LAUNCHED();
+    }
+    GX_CUDA(cudaStreamSynchronize(s));
+}
+
 void hash_join(const join_inputs& in, const gx_join_hint& hint, bool rowids_only, cudaStream_t s, gx_table* out) {
     const sides sd = pick_sides(in);
     const int kw = size_of(in.lkey.type), kind = vkind_of(in.lkey.type);
-    const int64_t nb = sd.bkey->n, np = sd.pkey->n;
+    const int64_t nb = sd.bkey->n;
     require(nb < (int64_t)0x7FFFFFFF, "hash join: the build side (smaller input) must have fewer than 2^31 rows");
     // Unique integer build keys: one probe pass instead of count and write.
-    if (unique_hash_join(in, hint, rowids_only, sd.build_left, s, out)) return;
+    key_table dup;
+    if (unique_hash_join(in, hint, rowids_only, sd.build_left, s, out, &dup)) return;
+    if (dup.width) {
+        const unsigned long long* t = dup.slots.get<unsigned long long>();
+        if (dup.width == 8) hj_join(slot_table<4, 8>{t, dup.mask}, in, sd, hint, rowids_only, dup.pay_in_run, s, out);
+        else if (kw == 4) hj_join(slot_table<4, 16>{t, dup.mask}, in, sd, hint, rowids_only, dup.pay_in_run, s, out);
+        else hj_join(slot_table<8, 16>{t, dup.mask}, in, sd, hint, rowids_only, dup.pay_in_run, s, out);
+        return;
+    }
     const uint64_t cap = next_pow2((uint64_t)std::max<int64_t>(64, 2 * nb));
     const int64_t words = (int64_t)cap * (kw == 4 ? 1 : 2);
     dbuf table((size_t)words * 8, s);
@@ -264,28 +326,9 @@ void hash_join(const join_inputs& in, const gx_join_hint& hint, bool rowids_only
         else k_hj_build<8><<<grid_for(nb, 256, 8), 256, 0, s>>>(sd.bkey->data, nb, kind, table.get<unsigned long long>(), cap - 1);
         GX_LAUNCHED();
     }
-    const int64_t ntiles = ceil_div(std::max<int64_t>(np, 1), HJ_TILE);
-    dbuf tc((size_t)ntiles * 8, s), toff((size_t)(ntiles + 1) * 8, s);
-    int64_t total = 0;
-    join_out none;
-    std::memset(&none, 0, sizeof(none));
-    if (np > 0 && nb > 0) {
-        GX_PROF("join_probe_count", s);
-        if (kw == 4) k_hj_probe<4, false><<<(unsigned)ntiles, HJ_NT, 0, s>>>(table.get<unsigned long long>(), cap - 1, sd.pkey->data, np, kind, tc.get<int64_t>(), nullptr, none);
-        else k_hj_probe<8, false><<<(unsigned)ntiles, HJ_NT, 0, s>>>(table.get<unsigned long long>(), cap - 1, sd.pkey->data, np, kind, tc.get<int64_t>(), nullptr, none);
-        GX_LAUNCHED();
-        exclusive_scan_i64(tc.get<int64_t>(), toff.get<int64_t>(), ntiles, s);
-        total = read_scalar(toff.get<int64_t>() + ntiles, s);
-    }
-    check_max_out(hint, total);
-    join_out o = make_outputs(in, sd.build_left, rowids_only, false, true, total, s, out);
-    if (total > 0) {
-        GX_PROF("join_probe_write", s);
-        if (kw == 4) k_hj_probe<4, true><<<(unsigned)ntiles, HJ_NT, 0, s>>>(table.get<unsigned long long>(), cap - 1, sd.pkey->data, np, kind, nullptr, toff.get<int64_t>(), o);
-        else k_hj_probe<8, true><<<(unsigned)ntiles, HJ_NT, 0, s>>>(table.get<unsigned long long>(), cap - 1, sd.pkey->data, np, kind, nullptr, toff.get<int64_t>(), o);
-        GX_LAUNCHED();
-    }
-    GX_CUDA(cudaStreamSynchronize(s));
+    const unsigned long long* t = table.get<unsigned long long>();
+    if (kw == 4) hj_join(record_table<4>{t, cap - 1}, in, sd, hint, rowids_only, false, s, out);
+    else hj_join(record_table<8>{t, cap - 1}, in, sd, hint, rowids_only, false, s, out);
 }
 
 void partition_hash_join(const join_inputs& in, const gx_join_hint& hint, bool rowids_only, cudaStream_t s,

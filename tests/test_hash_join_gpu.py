@@ -216,3 +216,40 @@ def test_selective_join_is_written_when_it_returns(algo, form, npr, share):
             for c in range(n_pay):
                 assert np.array_equal(cols[2 + c], pays[c][want_p].cpu().numpy())
         del t
+
+
+@pytest.mark.parametrize("kdt", [np.int32, np.uint32, np.int64, np.uint64])
+@pytest.mark.parametrize("nb,npr", [(2, 7), (900, 2049), (40_000, 50_001), (4_000, (1 << 20) + 5)])
+@pytest.mark.parametrize("marker", [False, True])
+def test_duplicate_build_keys_in_the_key_table(kdt, nb, npr, marker):
+    # Duplicated integer keys are probed in the table that was built to find
+    # out whether they are unique, below and above the size at which a probe is
+    # queued before that is known: row ids, one payload (held in the slots) of 4
+    # and 8 bytes, a narrow one, and two.  Keys at the type's limits, and with
+    # `marker` the 8-byte key that marks empty slots (another table then).
+    rng = np.random.default_rng(nb)
+    lim = np.iinfo(kdt)
+    edge = np.array([lim.max, lim.min, lim.max - 1, 0], kdt)
+    if np.dtype(kdt).itemsize == 8 and not marker:
+        edge = edge[edge.view(np.uint64) != np.uint64(2**63)]
+    elif marker:
+        edge = np.append(edge, np.array([-2**63 if np.dtype(kdt).itemsize == 8 else -2**31], np.int64).astype(kdt))
+    pool = np.concatenate([edge, rng.integers(1, lim.max - 1, nb, dtype=kdt)])
+    bk = rng.choice(pool[: max(2, nb // 2)], nb)
+    bk[-1] = bk[0]
+    pk = rng.choice(np.concatenate([pool, rng.integers(1, lim.max - 1, nb, dtype=kdt)]), npr)
+    el, er = O.join_pairs(bk, pk)
+    l, r = rowid_pairs(bk, pk, gx.JOIN_HASH)
+    assert np.array_equal(l, el) and np.array_equal(r, er)
+    pp = np.arange(npr)
+    for pdts in ((np.int64,), (np.float32,), (np.int16,), (np.int64, np.int32)):
+        bps = [(np.arange(nb) * (c + 1)).astype(d) for c, d in enumerate(pdts)]
+        t = gx.inner_eq_join([to_dev(bk), *map(to_dev, bps)], [to_dev(pk), to_dev(pp)],
+                             gx.make_join_hint(gx.JOIN_HASH, gx.MAT_GFUR))
+        cols = t.numpy_columns()
+        key, b, p = cols[0], cols[1:-1], cols[-1]
+        assert np.array_equal(key, pk[p])
+        o, e = np.lexsort((*b, p)), np.lexsort((*[x[el] for x in bps], er))
+        assert np.array_equal(p[o], er[e])
+        for got, x in zip(b, bps):
+            assert np.array_equal(got[o], x[el][e])
