@@ -58,8 +58,9 @@ struct key_table {
 
 // One-pass join of unique integer build keys through a hash table (gx_join.cu).
 // Returns false, with no output, when the build keys are not unique integers
-// or memory is short: the caller takes another plan.  With `dup`, a table whose
-// keys are not unique is completed and left there if it fits in L2.
+// or memory is short: the caller takes another plan.  A HASH join gives `dup`:
+// a table whose keys are not unique is completed and left there if it fits in
+// L2, and the outputs of a long probe are sized by its matches.
 bool unique_hash_join(const join_inputs& in, const gx_join_hint& hint, bool rowids_only, bool build_left,
                       cudaStream_t s, gx_table* out, key_table* dup = nullptr);
 

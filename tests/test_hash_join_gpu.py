@@ -4,6 +4,8 @@ duplicate keys on both sides, a hot build key that overflows one
 partition's shared-memory table (taken in chunks), float keys where -0.0
 equals +0.0, sizes that need two radix passes, wide payloads and empty
 sides.  Pairs are compared after sorting by (left row, right row)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -14,6 +16,12 @@ from tests.helpers import to_dev
 pytestmark = pytest.mark.gpu
 
 ALGOS = [gx.JOIN_HASH, gx.JOIN_PARTITION]
+
+
+def mem_stats():
+    cur, peak = C.c_int64(), C.c_int64()
+    gx.check(gx.lib.gx_mem_stats(C.byref(cur), C.byref(peak)))
+    return cur.value, peak.value
 
 
 def rowid_pairs(lk, rk, algo, **kw):
@@ -253,3 +261,62 @@ def test_duplicate_build_keys_in_the_key_table(kdt, nb, npr, marker):
         assert np.array_equal(p[o], er[e])
         for got, x in zip(b, bps):
             assert np.array_equal(got[o], x[el][e])
+
+
+@pytest.mark.parametrize("kdt", [np.int32, np.int64])
+@pytest.mark.parametrize("share", [0.0, 0.01, 0.5, 1.0])
+def test_hash_join_outputs_follow_the_matches(kdt, share):
+    # A long probe's outputs have room for the matches that a sample predicts,
+    # not for every probe row.
+    import torch
+    nb, npr, step, n_pay = 50_021, (1 << 22) + 1, 10_007, 5
+    t = torch.int32 if kdt == np.int32 else torch.int64
+    g = torch.Generator(device="cuda")
+    g.manual_seed(3)
+    ids = torch.randperm(nb, device="cuda", generator=g)
+    pid = torch.randint(0, nb, (npr,), device="cuda", generator=g)
+    miss = torch.rand(npr, device="cuda", generator=g) >= share
+    bk, pk = (ids * step).to(t), (pid * step + miss.long()).to(t)
+    pays = [pid * (c + 1) for c in range(n_pay)]
+    torch.cuda.synchronize()
+    current, _ = mem_stats()
+    gx.check(gx.lib.gx_mem_reset_peak())
+    out = gx.inner_eq_join([bk, ids], [pk, *pays], gx.make_join_hint(gx.JOIN_HASH, gx.MAT_GFUR))
+    _, peak = mem_stats()
+    width = np.dtype(kdt).itemsize + 8 * (n_pay + 1)
+    # A table of 2^17 slots of 16 bytes, tile states, and 1.2% of the rows to
+    # spare in each column.
+    assert peak - current <= (share + 0.012) * npr * width + (4 << 20)
+    want = torch.nonzero(~miss).squeeze(1)
+    assert out.num_rows == want.numel()
+    cols = out.numpy_columns()
+    assert np.array_equal(cols[0], pk[want].cpu().numpy()) and np.array_equal(cols[1], pid[want].cpu().numpy())
+    for c in range(n_pay):
+        assert np.array_equal(cols[2 + c], pays[c][want].cpu().numpy())
+
+
+@pytest.mark.parametrize("kdt", [np.int32, np.int64])
+@pytest.mark.parametrize("pay", [False, True])
+def test_matches_that_the_sample_misses(kdt, pay):
+    # Every row matches but the ones that the size of the outputs is sampled
+    # from: the probe runs again with room for all.
+    nb, npr, step = 4099, (1 << 22) + 77, 10_007
+    rng = np.random.default_rng(9)
+    ids = rng.permutation(nb)
+    pid = rng.integers(0, nb, npr)
+    i = np.arange(1 << 15, dtype=np.uint64)
+    every = npr // (1 << 15)
+    miss = np.zeros(npr, bool)
+    miss[(i * every + (i * 2654435761 % 2**32) % every).astype(np.int64)] = True
+    bk, pk = (ids * step).astype(kdt), (pid * step + miss).astype(kdt)
+    want = np.nonzero(~miss)[0]
+    row_of = np.empty(nb, np.int64)
+    row_of[ids] = np.arange(nb)
+    hint = gx.make_join_hint(gx.JOIN_HASH, gx.MAT_GFUR)
+    if pay:
+        out = gx.inner_eq_join([to_dev(bk), to_dev(ids)], [to_dev(pk), to_dev(pid)], hint)
+        key, b, p = out.numpy_columns()
+        assert np.array_equal(key, pk[want]) and np.array_equal(b, pid[want]) and np.array_equal(p, pid[want])
+    else:
+        b, p = gx.inner_eq_join_rowids(to_dev(bk), to_dev(pk), hint).numpy_columns()
+        assert np.array_equal(b, row_of[pid[want]]) and np.array_equal(p, want)
