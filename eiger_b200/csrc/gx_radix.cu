@@ -449,6 +449,7 @@ __global__ void __launch_bounds__(OH_NT, 2) k_radix_hist_all(const void* __restr
 // lane) order: the lanes of a digit find each other through a shared bit mask
 // (one atomicOr and one read), the highest of them adds their number to the
 // warp's count and clears the mask.  `wm` must be zero before the first call.
+// (The steps of the atomic-OR ranking in NVIDIA's open-source CUB radix sort.)
 // On B200 this costs 0.31 ms per 2^28 rows and digit where __match_any_sync
 // costs 1.8 ms and eight ballots 0.73 ms (16 warps per CTA, random digits).
 __device__ __forceinline__ unsigned warp_rank(unsigned* wm, unsigned* wh, unsigned d, bool valid, int lane) {
@@ -611,7 +612,27 @@ __global__ void __launch_bounds__(OS_NT, 2) k_radix_onesweep(digit_of<KW, FLT> d
 
     const int local0 = warp * 32 * IPT + lane;  // row (k, lane) of the warp: local0 + 32 k
     unsigned rk[IPT];  // digit << 16 | rank in the warp's rows of the digit
-    if (full) {
+    // Lanes with one digit queue on its word, so a warp whose first rows share a
+    // digit (ordered input, constant digits) looks for such rows and ranks them
+    // by lane.  2^25 int64 keys with int32 values into 16 parts, runs of 64 equal
+    // keys: 312 us a call, 395 without; 2^28 random int32 keys with int64 values:
+    // 8.22 ms, 8.20 without.
+    auto one_digit = [](unsigned d) { return (bool)__all_sync(0xffffffffu, d == __shfl_sync(0xffffffffu, d, 0)); };
+    if (full && one_digit(dg(row_key(local0)))) {
+#pragma unroll
+        for (int k = 0; k < IPT; ++k) {
+            const unsigned d = dg(row_key(local0 + 32 * k));
+            if (one_digit(d)) {
+                const unsigned prior = wh[d];
+                __syncwarp();
+                if (lane == 0) wh[d] = prior + 32;
+                __syncwarp();
+                rk[k] = (prior + lane) | d << 16;
+            } else {
+                rk[k] = warp_rank(wm, wh, d, true, lane) | d << 16;
+            }
+        }
+    } else if (full) {
 #pragma unroll
         for (int k = 0; k < IPT; ++k) {
             const unsigned d = dg(row_key(local0 + 32 * k));

@@ -104,6 +104,25 @@ def test_sort_one_cta_and_onesweep_edges(n, kdt, vdt):
         assert np.array_equal(idx.cpu().numpy(), ei)
 
 
+@pytest.mark.parametrize("n", [30_011, 18432 * 30 + 5])
+@pytest.mark.parametrize("kdt,vdt", [(np.int32, np.int64), (np.int64, np.int32), (np.int16, np.int64)])
+@pytest.mark.parametrize("run", [31, 32, 33, 100, 700])
+def test_sort_runs_of_equal_keys(n, kdt, vdt, run):
+    # Warps whose rows share a digit in some of their row groups, from the first
+    # one on or not, between groups of many digits.
+    rng = np.random.default_rng(run)
+    lim = np.iinfo(kdt)
+    starts = rng.integers(lim.min, lim.max, n // run + 1).astype(kdt)
+    k = np.repeat(starts, run)[:n]
+    mixed = rng.random(n) < 0.02 * (np.arange(n) // 1000 % 2)
+    k[mixed] = rng.integers(lim.min, lim.max, int(mixed.sum())).astype(kdt)
+    v = np.arange(n).astype(vdt)
+    for b, e, desc in ((0, -1, False), (4, 12, True)):
+        sk, sv = gx.sort_column_pair(to_dev(k), to_dev(v), b, e, gx.DESCENDING if desc else gx.ASCENDING)
+        ek, ev = O.sort_pairs(k, v, b, e, desc)
+        assert np.array_equal(sk.cpu().numpy(), ek) and np.array_equal(sv.cpu().numpy(), ev)
+
+
 @pytest.mark.parametrize("n", [50_000, 512 * 4 * 300 + 7, 4608 * 148 * 5 + 1])
 @pytest.mark.parametrize("kdt,vdt", [(np.int32, np.int64), (np.float64, np.int32), (np.int64, np.int64)])
 @pytest.mark.parametrize("off", [0, 1])
