@@ -237,33 +237,6 @@ __global__ void k_image_range(const void* __restrict__ keys, int64_t n, img_para
     }
 }
 
-// The same for up to IR_ONE keys in one CTA, which writes out[] itself.
-constexpr int64_t IR_ONE = 1 << 15;
-template <int KW>
-__global__ void __launch_bounds__(1024) k_image_range_one(const void* __restrict__ keys, int64_t n, img_params ip,
-                                                          unsigned long long* __restrict__ out) {
-    __shared__ unsigned long long s_lo[32], s_hi[32];
-    unsigned long long lo = ~0ull, hi = 0;
-    for (int64_t i = threadIdx.x; i < n; i += 1024) {
-        const uint64_t img = key_image<KW>(load_key<KW>(keys, i), ip);
-        lo = min(lo, (unsigned long long)img);
-        hi = max(hi, (unsigned long long)img);
-    }
-    for (int round = 0; round < 2; ++round) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-            hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-        }
-        if (round) break;
-        if ((threadIdx.x & 31) == 0) { s_lo[threadIdx.x >> 5] = lo; s_hi[threadIdx.x >> 5] = hi; }
-        __syncthreads();
-        lo = s_lo[threadIdx.x & 31];
-        hi = s_hi[threadIdx.x & 31];
-    }
-    if (threadIdx.x == 0) { out[0] = lo; out[1] = hi; }
-}
-
 template <typename S, typename D>
 __global__ void k_narrow(D* __restrict__ out, const S* __restrict__ in, int64_t n) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -988,19 +961,13 @@ void key_image_range(const col& keys, uint64_t* lo, uint64_t* hi, cudaStream_t s
     require(w == 4 || w == 8, "key_image_range: 4/8-byte keys only");
     img_params ip{vkind_of(keys.type), w, 0, 0};
     dbuf out(16, s);
-    if (keys.n > 0 && keys.n <= IR_ONE) {
-        if (w == 4) k_image_range_one<4><<<1, 1024, 0, s>>>(keys.data, keys.n, ip, out.get<unsigned long long>());
-        else k_image_range_one<8><<<1, 1024, 0, s>>>(keys.data, keys.n, ip, out.get<unsigned long long>());
+    GX_CUDA(cudaMemsetAsync(out.get(), 0xFF, 8, s));
+    GX_CUDA(cudaMemsetAsync(out.get<char>() + 8, 0, 8, s));
+    if (keys.n > 0) {
+        int g = grid_for(keys.n, 256, 8);
+        if (w == 4) k_image_range<4><<<g, 256, 0, s>>>(keys.data, keys.n, ip, out.get<unsigned long long>());
+        else k_image_range<8><<<g, 256, 0, s>>>(keys.data, keys.n, ip, out.get<unsigned long long>());
         GX_LAUNCHED();
-    } else {
-        GX_CUDA(cudaMemsetAsync(out.get(), 0xFF, 8, s));
-        GX_CUDA(cudaMemsetAsync(out.get<char>() + 8, 0, 8, s));
-        if (keys.n > 0) {
-            int g = grid_for(keys.n, 256, 8);
-            if (w == 4) k_image_range<4><<<g, 256, 0, s>>>(keys.data, keys.n, ip, out.get<unsigned long long>());
-            else k_image_range<8><<<g, 256, 0, s>>>(keys.data, keys.n, ip, out.get<unsigned long long>());
-            GX_LAUNCHED();
-        }
     }
     uint64_t h[2];
     host_read(h, out.get(), 16, s);
