@@ -155,11 +155,20 @@ void* thread_scratch(int slot, size_t bytes) {
 }
 
 namespace {
+// Pinned memory is taken and freed in the relaxed capture mode: in the default
+// one these calls fail while any thread captures a graph, and end its capture.
+struct relaxed_capture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    relaxed_capture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~relaxed_capture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
 // Pinned staging of host_read: one small buffer per host thread, freed with it.
 struct pinned_stage {
     void* p = nullptr;
     ~pinned_stage() {
-        if (p) cudaFreeHost(p);  // errors ignored: the context may already be gone at exit
+        if (!p) return;
+        relaxed_capture relaxed;
+        cudaFreeHost(p);  // errors ignored: the context may already be gone at exit
     }
 };
 thread_local pinned_stage t_stage;
@@ -167,7 +176,10 @@ thread_local pinned_stage t_stage;
 
 void host_read(void* dst, const void* dptr, size_t bytes, cudaStream_t s) {
     require(bytes <= HOST_READ_MAX, "host_read: too many bytes");
-    if (!t_stage.p) GX_CUDA(cudaHostAlloc(&t_stage.p, HOST_READ_MAX, cudaHostAllocPortable));
+    if (!t_stage.p) {
+        relaxed_capture relaxed;
+        GX_CUDA(cudaHostAlloc(&t_stage.p, HOST_READ_MAX, cudaHostAllocPortable));
+    }
     GX_CUDA(cudaMemcpyAsync(t_stage.p, dptr, bytes, cudaMemcpyDeviceToHost, s));
     GX_CUDA(cudaStreamSynchronize(s));
     std::memcpy(dst, t_stage.p, bytes);
