@@ -38,11 +38,10 @@ def test_sort_pairs_bit_exact(kdt, bits, desc):
 
 @pytest.mark.parametrize("per_tile", [False, True])
 @pytest.mark.parametrize("kdt,vdt", [(np.int32, np.int64), (np.float64, np.int32), (np.uint64, np.float64)])
-def test_sort_pairs_persistent_and_per_tile_passes(monkeypatch, per_tile, kdt, vdt):
-    # Several tiles per SM and a partial last tile, through the persistent
-    # bulk-copy digit passes and through the per-tile kernel
-    # (GX_RADIX_NO_BULK): both bit-exact, ascending and descending, on a bit
-    # range and on row ids.
+def test_sort_pairs_one_sweep_and_per_tile_passes(monkeypatch, per_tile, kdt, vdt):
+    # Several tiles per SM and a partial last tile, through the one-sweep
+    # passes and through the per-tile kernels (GX_RADIX_NO_BULK): both
+    # bit-exact, ascending and descending, on a bit range and on row ids.
     if per_tile:
         monkeypatch.setenv("GX_RADIX_NO_BULK", "1")
     n = 148 * 3 * 4096 + 1234
@@ -72,12 +71,15 @@ def test_argsort_and_sort_column(n):
     assert np.array_equal(only.cpu().numpy(), ek)
 
 
-@pytest.mark.parametrize("n", [2, 61, 255, 256, 257, 8191, 8192, 8193, 2048 * 7, 2048 * 7 + 1, (1 << 19) - 1, 1 << 19, 5120 * 149 + 3])
+@pytest.mark.parametrize("n", [2, 61, 255, 256, 257, 8191, 8192, 8193, 2048 * 7, 2048 * 7 + 1, (1 << 19) - 1, 1 << 19,
+                               18432 * 29 - 1, 18432 * 29, 18432 * 29 + 1, 8192 * 65 - 1, 8192 * 65 + 1, 5120 * 149 + 3])
 @pytest.mark.parametrize("kdt,vdt", [(np.int8, np.int64), (np.uint16, np.int32), (np.int32, np.int32),
                                      (np.float32, np.int64), (np.int64, np.int64), (np.float64, np.int32)])
 def test_sort_one_cta_and_onesweep_edges(n, kdt, vdt):
     # The counting sort (up to 256 rows), the one-CTA sort (up to 8192) and the
-    # look-back passes at the edges of their tiles, from views that start on and off 16-byte boundaries, with
+    # look-back passes at the edges of their tiles (2048 rows below 2^19; above,
+    # 4608 for 8 + 8 bytes, 6144 for 4 + 8 and 8 + 4, 8192 for the others; 18432
+    # is a multiple of the first two), from views that start on and off 16-byte boundaries, with
     # keys whose digits vary, are all the same in some passes (skipped) or in
     # all of them, as pairs and as row ids.
     rng = np.random.default_rng(n)
