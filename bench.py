@@ -354,9 +354,10 @@ def run_gx(args) -> None:
         for algo, nm in ((gx.JOIN_HASH, "hash"), (gx.JOIN_PARTITION, "partition_hash")):
             h3 = gx.make_join_hint(algo, gx.MAT_GFUR, unique_left=1)
             join[nm] = measure(lambda: gx.inner_eq_join_rowids(bk, pk, h3), lambda m: (nb + npr) * 4 + m * 16)
-        # The sorted-build matcher: the same join with keys spread 8 apart, so
-        # the build side is too sparse for direct placement; sorted build run
-        # + radix directory (SORTED_BUILD) and both sides sorted (SORT_MERGE).
+        # The same join with keys spread 8 apart, so the build side is too
+        # sparse for direct placement: sort_mode SORTED_BUILD (unique keys, as
+        # here, go through a hash table; others through a sorted run and its
+        # radix directory) and both sides sorted (SORT_MERGE).
         sbk, spk = bk * 8, pk * 8
         for mode, nm in ((gx.SORTED_BUILD, "sorted_build"), (gx.SORT_MERGE, "sort_merge")):
             h2 = gx.make_join_hint(gx.JOIN_SORT, gx.MAT_GFUR, unique_left=1, sort_mode=mode)
@@ -777,8 +778,8 @@ def main() -> None:
     ap.add_argument("--join-only", action="store_true", help="only the rowid join (profiling captures)")
     ap.add_argument("--join-mode", default="auto", choices=["auto", "sorted_build", "sort_merge", "hash",
                                                              "partition_hash"],
-                    help="matcher of --join-only: auto (dense placement when the build keys allow it), the "
-                         "sorted-build or sort-merge matcher on keys spread 8 apart, or the hash joins")
+                    help="matcher of --join-only: auto (dense placement when the build keys allow it), sort_mode "
+                         "SORTED_BUILD or SORT_MERGE on keys spread 8 apart, or the hash joins")
     ap.add_argument("--selector", choices=["learned", "plain"], default="learned",
                     help="AUTO's chooser: the learned FP16 MLP (committed weights) or the plain NDV rule")
     ap.add_argument("--batch-instances", type=int, default=512, help="batched pipeline instances (0: skip)")

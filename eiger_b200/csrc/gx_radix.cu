@@ -491,10 +491,10 @@ constexpr int os_ipt_max() {
 // back for the start of its digit runs; then output position j fetches its
 // row's key and value from shared memory and writes them, run by run.
 // Bound by shared-memory wavefronts (about 40 per 32 rows: the rank, the list
-// and the gathers are random accesses; L1 71% busy, HBM 38%).  2^28 random
-// rows per pass, measured over a whole sort: 2.05 ms for int32 keys with int64
+// and the gathers are random accesses; L1 70% busy, HBM 38%).  2^28 random
+// rows per pass, measured over a whole sort: 1.95 ms for int32 keys with int64
 // values (3.5 ms with the stable ranking by __match_any_sync, plus 0.9 ms of
-// counting per pass), 1.7 ms for int32 with int32, 2.7 ms for int64 with int64.
+// counting per pass), 1.6 ms for int32 with int32, 2.45 ms for int64 with int64.
 // Two CTAs of 512 threads with 6144 rows beat three of 4608 rows (9.05 against
 // 10.6 ms a sort), one of 1024 threads (9.6 ms) and 768 threads (10.6 ms); a
 // look-back window of 8 tiles beats 4 and 16 by 3% and 10%.
